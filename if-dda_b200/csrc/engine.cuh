@@ -192,6 +192,17 @@ template <class T, class Pre, class Epi>
 bool matvec_launch_fused(const MvArgs<T>& a, const Pre& pre, const Epi& epi, const MvRed& red, int nrhs, bool tab,
                          cudaStream_t st);
 
+// Passes 2 to 4 (y, zconv, y) of nrhs right-hand sides.
+template <class T> void launch_yz(const MvArgs<T>& a, int nrhs, cudaStream_t st);
+
+// brackets one pass launch with the optional timing events and counts it
+struct PassScope {
+    cudaEvent_t ev;
+    cudaStream_t st;
+    PassScope(int pass, int bytes, cudaStream_t s) : ev(timing_before(pass, bytes, s)), st(s) { count_launch(); }
+    ~PassScope() { timing_after(ev, st); }
+};
+
 // fill MvArgs from a Green object and the caller's vectors
 template <class T>
 MvArgs<T> mv_args(Green& G, int nrhs, const cplx<T>* x, const cplx<T>* b, cplx<T>* y, long xstride, int amode,

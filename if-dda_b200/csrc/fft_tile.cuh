@@ -5,8 +5,10 @@
 //     v[r] = x[j + r L/R] * w^(DIR * (j mod Ns) * r * L / (Ns R)),  r < R
 //     v    = DFT_R(v, DIR)
 //     x[(j / Ns) Ns R + (j mod Ns) + r Ns] = v[r]
-// Every thread keeps its butterflies in registers across a barrier, so the
-// transform runs in place.  DIR = +1 is exp(+i 2 pi jk / L) (the reference's
+// An inner pass keeps its butterflies in registers across a barrier, so the
+// transform runs in place; a pass that reads from global memory or writes to
+// it has no such hazard and no barrier of its own (after a transform that ends
+// in global memory, a caller that reuses the tile synchronises first).  DIR = +1 is exp(+i 2 pi jk / L) (the reference's
 // "forward" convention for G and x, cdmlib/calculgreenfft.f:16,76-99), DIR = -1
 // the inverse; both unnormalised.  L may be any product of 2, 3 and 5.
 //
@@ -61,18 +63,122 @@ __host__ __device__ constexpr int clamp_pow2(int v, int lo, int hi) {
 }
 // Radices with a register butterfly (Dft<R> below).
 __host__ __device__ constexpr bool has_dft(int r) {
-    return r == 2 || r == 3 || r == 4 || r == 5 || r == 8 || r == 12 || r == 16 || r == 32;
+    return r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 8 || r == 10 || r == 12 || r == 16 || r == 32;
 }
-// Plan policy 1 (two passes): a first radix of 32 or 16 and one more radix of
-// at most 12, where such a pair exists; otherwise policy 0.  It halves the
-// shared-memory round trips of a three-pass length (160, 192, 256, 384) for
-// a kernel that can afford the registers of a 32-point butterfly.
-__host__ __device__ constexpr int two_pass_first(int L) {
-    return (L % 32 == 0 && has_dft(L / 32) && L / 32 <= 12) ? 32
-         : (L % 16 == 0 && has_dft(L / 16) && L / 16 <= 12) ? 16 : 0;
+// Plans of the mat-vec passes (policy 0 is the general rule above):
+//  PLAN_Z: two passes up to 384, the second (whose butterflies hold all three
+//      components of a column in registers) of at most 8 points up to 256 and
+//      12 above: 16-byte elements at three times 8 points take 96 registers;
+//  PLAN_Z3: three passes with small radices: one shared-memory round trip more
+//      per direction, for half the registers and twice the warps;
+//  PLAN_Y: two passes up to 512;
+//  PLAN_X: the last radix is even and at most 12, since a thread of the last
+//      forward (first inverse) pass holds two butterflies at once.
+enum { PLAN_ANY = 0, PLAN_Z = 1, PLAN_Y = 2, PLAN_X = 3, PLAN_Z3 = 4 };
+struct RadixPlan {
+    int r[3];
+};
+__host__ __device__ constexpr RadixPlan plan_table(int L, int policy) {
+    switch (policy) {
+    case PLAN_Z:
+        switch (L) {
+        case 4: return {{2, 2}};
+        case 6: return {{2, 3}};
+        case 8: return {{4, 2}};
+        case 10: return {{2, 5}};
+        case 12: return {{4, 3}};
+        case 16: return {{4, 4}};
+        case 20: return {{4, 5}};
+        case 24: return {{8, 3}};
+        case 32: return {{8, 4}};
+        case 40: return {{8, 5}};
+        case 48: return {{16, 3}};
+        case 64: return {{16, 4}};
+        case 80: return {{16, 5}};
+        case 96: return {{16, 6}};
+        case 128: return {{16, 8}};
+        case 160: return {{32, 5}};
+        case 192: return {{32, 6}};
+        case 256: return {{32, 8}};
+        case 320: return {{32, 10}};
+        case 384: return {{32, 12}};
+        case 512: return {{16, 8, 4}};
+        case 640: return {{16, 8, 5}};
+        }
+        break;
+    case PLAN_Z3:
+        switch (L) {
+        case 160: return {{8, 5, 4}};
+        case 192: return {{8, 6, 4}};
+        case 256: return {{8, 8, 4}};
+        case 320: return {{8, 10, 4}};
+        case 384: return {{8, 12, 4}};
+        case 512: return {{8, 16, 4}};
+        case 640: return {{16, 10, 4}};
+        }
+        break;
+    case PLAN_Y:
+        switch (L) {
+        case 6: return {{6}};
+        case 10: return {{10}};
+        case 12: return {{12}};
+        case 16: return {{16}};
+        case 20: return {{4, 5}};
+        case 24: return {{8, 3}};
+        case 32: return {{8, 4}};
+        case 40: return {{8, 5}};
+        case 48: return {{8, 6}};
+        case 64: return {{8, 8}};
+        case 80: return {{8, 10}};
+        case 96: return {{16, 6}};
+        case 128: return {{16, 8}};
+        case 160: return {{16, 10}};
+        case 192: return {{16, 12}};
+        case 256: return {{16, 16}};
+        case 320: return {{32, 10}};
+        case 384: return {{32, 12}};
+        case 512: return {{32, 16}};
+        case 640: return {{16, 8, 5}};
+        }
+        break;
+    case PLAN_X:
+        switch (L) {
+        case 4: return {{2, 2}};
+        case 6: return {{3, 2}};
+        case 8: return {{2, 4}};
+        case 10: return {{5, 2}};
+        case 12: return {{3, 4}};
+        case 16: return {{4, 4}};
+        case 20: return {{5, 4}};
+        case 24: return {{3, 8}};
+        case 32: return {{4, 8}};
+        case 40: return {{5, 8}};
+        case 48: return {{6, 8}};
+        case 64: return {{8, 8}};
+        case 80: return {{10, 8}};
+        case 96: return {{16, 6}};
+        case 128: return {{16, 8}};
+        case 160: return {{16, 10}};
+        case 192: return {{16, 12}};
+        case 256: return {{4, 8, 8}};
+        case 320: return {{5, 8, 8}};
+        case 384: return {{16, 3, 8}};
+        case 512: return {{8, 8, 8}};
+        case 640: return {{10, 8, 8}};
+        }
+        break;
+    }
+    return {{0}};
 }
 __host__ __device__ constexpr int pick_radix_p(int L, int rem, bool first, int policy) {
-    if (policy == 1 && two_pass_first(L)) return first ? two_pass_first(L) : rem;
+    if (policy) {
+        const RadixPlan t = plan_table(L, policy);
+        int left = L;
+        for (int q = 0; q < 3 && t.r[q] > 0; q++) {
+            if (left == rem) return t.r[q];
+            left /= t.r[q];
+        }
+    }
     return pick_radix(rem, first);
 }
 // The plan of L: radix of pass q (0-based) and number of passes.  A plan
@@ -126,6 +232,10 @@ __host__ __device__ constexpr int max_radix(int L, int policy = 0) {
 #define IFDDA_S1_5 0.95105651629515357211643933337938   // sin(2 pi / 5)
 #define IFDDA_S2_5 0.58778525229247312916870595463907   // sin(4 pi / 5)
 
+// Butterflies, in place on registers.  C is an FFT element (float2, double2
+// or cpair); run_half assumes v[r] = 0 for r >= R / 2 (the padding), whose
+// sums it leaves out.  Composite radices with coprime factors (6, 10, 12) use
+// the prime-factor index maps, which need no inner twiddles.
 template <int R, int DIR, class C> struct Dft;
 
 template <int DIR, class C> struct Dft<2, DIR, C> {
@@ -134,40 +244,125 @@ template <int DIR, class C> struct Dft<2, DIR, C> {
         v[0] = cadd(a, b);
         v[1] = csub(a, b);
     }
+    __device__ __forceinline__ static void run_half(C* v) { v[1] = v[0]; }
+};
+
+template <int DIR, class C> struct Dft<3, DIR, C> {
+    __device__ __forceinline__ static void run(C* v) {
+        using T = typename elem_traits<C>::T;
+        C t1 = cadd(v[1], v[2]);
+        C t2 = cfma_s(v[0], t1, (T)-0.5);
+        C t3 = csub(v[1], v[2]);
+        const T s = DIR > 0 ? (T)IFDDA_SQRT3_2 : (T)-IFDDA_SQRT3_2;
+        v[0] = cadd(v[0], t1);
+        v[1] = cfma_i(t2, t3, s);
+        v[2] = cfma_i(t2, t3, -s);
+    }
 };
 
 template <int DIR, class C> struct Dft<4, DIR, C> {
     __device__ __forceinline__ static void run(C* v) {
         C s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-        C s13 = cadd(v[1], v[3]), d13 = cmul_i<DIR>(csub(v[1], v[3]));
+        C s13 = cadd(v[1], v[3]), d13 = csub(v[1], v[3]);
         v[0] = cadd(s02, s13);
         v[2] = csub(s02, s13);
-        v[1] = cadd(d02, d13);
-        v[3] = csub(d02, d13);
+        v[1] = cadd_i<DIR>(d02, d13);
+        v[3] = cadd_i<-DIR>(d02, d13);
+    }
+    __device__ __forceinline__ static void run_half(C* v) {
+        C a = v[0], b = v[1];
+        v[0] = cadd(a, b);
+        v[2] = csub(a, b);
+        v[1] = cadd_i<DIR>(a, b);
+        v[3] = cadd_i<-DIR>(a, b);
     }
 };
 
-template <int DIR, class C> struct Dft<8, DIR, C> {
+template <int DIR, class C> struct Dft<5, DIR, C> {
     __device__ __forceinline__ static void run(C* v) {
-        using T = decltype(C().x);
+        using T = typename elem_traits<C>::T;
+        const T c1 = (T)IFDDA_C1_5, c2 = (T)IFDDA_C2_5, s1 = (T)IFDDA_S1_5, s2 = (T)IFDDA_S2_5;
+        C t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
+        C t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
+        C a1 = cfma_s(cfma_s(v[0], t1, c1), t2, c2);
+        C a2 = cfma_s(cfma_s(v[0], t1, c2), t2, c1);
+        C b1 = cfma_s(cscale(t3, s1), t4, s2);
+        C b2 = cfma_s(cscale(t3, s2), t4, -s1);
+        v[0] = cadd(v[0], cadd(t1, t2));
+        v[1] = cadd_i<DIR>(a1, b1);
+        v[4] = cadd_i<-DIR>(a1, b1);
+        v[2] = cadd_i<DIR>(a2, b2);
+        v[3] = cadd_i<-DIR>(a2, b2);
+    }
+};
+
+// A x B points, A and B coprime: X[(n1 ka + n2 kb) mod R] from DFT_A over
+// DFT_B of x[(B n1 + A n2) mod R]; ka = 1 mod A and 0 mod B, kb the other way
+template <int A, int B, int DIR, class C> struct DftPfa {
+    static constexpr int R = A * B;
+    static constexpr int unit(int m, int n) {  // the multiple of n that is 1 mod m
+        int q = n;
+        while (q % m != 1) q += n;
+        return q;
+    }
+    __device__ __forceinline__ static void run(C* v) {
+        constexpr int ka = unit(A, B), kb = unit(B, A);
+        C a[A][B];
+#pragma unroll
+        for (int n1 = 0; n1 < A; n1++) {
+            C t[B];
+#pragma unroll
+            for (int n2 = 0; n2 < B; n2++) t[n2] = v[(B * n1 + A * n2) % R];
+            Dft<B, DIR, C>::run(t);
+#pragma unroll
+            for (int n2 = 0; n2 < B; n2++) a[n1][n2] = t[n2];
+        }
+#pragma unroll
+        for (int k2 = 0; k2 < B; k2++) {
+            C t[A];
+#pragma unroll
+            for (int n1 = 0; n1 < A; n1++) t[n1] = a[n1][k2];
+            Dft<A, DIR, C>::run(t);
+#pragma unroll
+            for (int k1 = 0; k1 < A; k1++) v[(k1 * ka + k2 * kb) % R] = t[k1];
+        }
+    }
+    __device__ __forceinline__ static void run_half(C* v) {
+#pragma unroll
+        for (int r = R / 2; r < R; r++) v[r] = czero<C>();
+        run(v);
+    }
+};
+template <int DIR, class C> struct Dft<6, DIR, C> : DftPfa<2, 3, DIR, C> {};
+template <int DIR, class C> struct Dft<10, DIR, C> : DftPfa<2, 5, DIR, C> {};
+template <int DIR, class C> struct Dft<12, DIR, C> : DftPfa<4, 3, DIR, C> {};
+
+template <int DIR, class C> struct Dft<8, DIR, C> {
+    template <bool HALF> __device__ __forceinline__ static void go(C* v) {
+        using T = typename elem_traits<C>::T;
         C e[4] = {v[0], v[2], v[4], v[6]};
         C o[4] = {v[1], v[3], v[5], v[7]};
-        Dft<4, DIR, C>::run(e);
-        Dft<4, DIR, C>::run(o);
+        if constexpr (HALF) {
+            Dft<4, DIR, C>::run_half(e);
+            Dft<4, DIR, C>::run_half(o);
+        } else {
+            Dft<4, DIR, C>::run(e);
+            Dft<4, DIR, C>::run(o);
+        }
         const T h = (T)IFDDA_SQRT1_2;
         // w^1 = (1 + DIR i)/sqrt2, w^2 = DIR i, w^3 = (-1 + DIR i)/sqrt2
-        C o1 = cscale(cadd(o[1], cmul_i<DIR>(o[1])), h);
-        C o2 = cmul_i<DIR>(o[2]);
-        C o3 = cscale(csub(cmul_i<DIR>(o[3]), o[3]), h);
+        const C o1 = cadd_i<DIR>(o[1], o[1]), o3 = cadd_i<-DIR>(o[3], o[3]);
         v[0] = cadd(e[0], o[0]);
         v[4] = csub(e[0], o[0]);
-        v[1] = cadd(e[1], o1);
-        v[5] = csub(e[1], o1);
-        v[2] = cadd(e[2], o2);
-        v[6] = csub(e[2], o2);
-        v[3] = cadd(e[3], o3);
-        v[7] = csub(e[3], o3);
+        v[1] = cfma_s(e[1], o1, h);
+        v[5] = cfma_s(e[1], o1, -h);
+        v[2] = cadd_i<DIR>(e[2], o[2]);
+        v[6] = cadd_i<-DIR>(e[2], o[2]);
+        v[3] = cfma_s(e[3], o3, -h);
+        v[7] = cfma_s(e[3], o3, h);
     }
+    __device__ __forceinline__ static void run(C* v) { go<false>(v); }
+    __device__ __forceinline__ static void run_half(C* v) { go<true>(v); }
 };
 
 // 16 points as 4 x 4: DFT4 over the stride-4 subsequences, the inner twiddles
@@ -175,13 +370,14 @@ template <int DIR, class C> struct Dft<8, DIR, C> {
 #define IFDDA_COS_PI8 0.92387953251128675612818318939679  // cos(pi / 8)
 #define IFDDA_SIN_PI8 0.38268343236508977172845998403040  // sin(pi / 8)
 template <int DIR, class C> struct Dft<16, DIR, C> {
-    __device__ __forceinline__ static void run(C* v) {
-        using T = decltype(C().x);
+    template <bool HALF> __device__ __forceinline__ static void go(C* v) {
+        using T = typename elem_traits<C>::T;
         C a[4][4];
 #pragma unroll
         for (int n2 = 0; n2 < 4; n2++) {
             C t[4] = {v[n2], v[4 + n2], v[8 + n2], v[12 + n2]};
-            Dft<4, DIR, C>::run(t);
+            if constexpr (HALF) Dft<4, DIR, C>::run_half(t);
+            else Dft<4, DIR, C>::run(t);
 #pragma unroll
             for (int k1 = 0; k1 < 4; k1++) a[n2][k1] = t[k1];
         }
@@ -189,24 +385,28 @@ template <int DIR, class C> struct Dft<16, DIR, C> {
         const T ds = DIR > 0 ? s : -s, dc = DIR > 0 ? c : -c, dh = DIR > 0 ? h : -h;
         // w^1 = c + i DIR s, w^2 = (1 + i DIR)/sqrt2, w^3 = s + i DIR c,
         // w^4 = i DIR, w^6 = (-1 + i DIR)/sqrt2, w^9 = -w^1
-        const C w1 = mk(c, ds), w2 = mk(h, dh), w3 = mk(s, dc), w6 = mk(-h, dh), w9 = mk(-c, -ds);
-        a[1][1] = cmul(a[1][1], w1);
-        a[1][2] = cmul(a[1][2], w2);
-        a[1][3] = cmul(a[1][3], w3);
-        a[2][1] = cmul(a[2][1], w2);
-        a[2][2] = cmul_i<DIR>(a[2][2]);
-        a[2][3] = cmul(a[2][3], w6);
-        a[3][1] = cmul(a[3][1], w3);
-        a[3][2] = cmul(a[3][2], w6);
-        a[3][3] = cmul(a[3][3], w9);
+        a[1][1] = cmulk(a[1][1], c, ds);
+        a[1][2] = cmulk(a[1][2], h, dh);
+        a[1][3] = cmulk(a[1][3], s, dc);
+        a[2][1] = cmulk(a[2][1], h, dh);
+        a[2][3] = cmulk(a[2][3], -h, dh);
+        a[3][1] = cmulk(a[3][1], s, dc);
+        a[3][2] = cmulk(a[3][2], -h, dh);
+        a[3][3] = cmulk(a[3][3], -c, -ds);
 #pragma unroll
         for (int k1 = 0; k1 < 4; k1++) {
-            C t[4] = {a[0][k1], a[1][k1], a[2][k1], a[3][k1]};
-            Dft<4, DIR, C>::run(t);
-#pragma unroll
-            for (int k2 = 0; k2 < 4; k2++) v[k1 + 4 * k2] = t[k2];
+            // the factor w^4 = i DIR of a[2][2] goes into its two sums
+            const C s02 = k1 == 2 ? cadd_i<DIR>(a[0][k1], a[2][k1]) : cadd(a[0][k1], a[2][k1]);
+            const C d02 = k1 == 2 ? cadd_i<-DIR>(a[0][k1], a[2][k1]) : csub(a[0][k1], a[2][k1]);
+            const C s13 = cadd(a[1][k1], a[3][k1]), d13 = csub(a[1][k1], a[3][k1]);
+            v[k1] = cadd(s02, s13);
+            v[k1 + 8] = csub(s02, s13);
+            v[k1 + 4] = cadd_i<DIR>(d02, d13);
+            v[k1 + 12] = cadd_i<-DIR>(d02, d13);
         }
     }
+    __device__ __forceinline__ static void run(C* v) { go<false>(v); }
+    __device__ __forceinline__ static void run_half(C* v) { go<true>(v); }
 };
 
 // 32 points as 2 x 16: DFT16 over the even and the odd points, the twiddles
@@ -216,95 +416,42 @@ template <int DIR, class C> struct Dft<16, DIR, C> {
 #define IFDDA_COS_3PI16 0.83146961230254523707878837761791  // cos(3 pi / 16)
 #define IFDDA_SIN_3PI16 0.55557023301960222474283081394853  // sin(3 pi / 16)
 template <int DIR, class C> struct Dft<32, DIR, C> {
-    __device__ __forceinline__ static void run(C* v) {
-        using T = decltype(C().x);
+    template <bool HALF> __device__ __forceinline__ static void go(C* v) {
+        using T = typename elem_traits<C>::T;
         C e[16], o[16];
 #pragma unroll
         for (int n = 0; n < 16; n++) {
             e[n] = v[2 * n];
             o[n] = v[2 * n + 1];
         }
-        Dft<16, DIR, C>::run(e);
-        Dft<16, DIR, C>::run(o);
+        if constexpr (HALF) {
+            Dft<16, DIR, C>::run_half(e);
+            Dft<16, DIR, C>::run_half(o);
+        } else {
+            Dft<16, DIR, C>::run(e);
+            Dft<16, DIR, C>::run(o);
+        }
         // cos and sin of k pi / 16, k = 0..8 (k pi / 16 for k > 8 by symmetry)
         const T cs[9] = {(T)1, (T)IFDDA_COS_PI16, (T)IFDDA_COS_PI8, (T)IFDDA_COS_3PI16, (T)IFDDA_SQRT1_2,
                          (T)IFDDA_SIN_3PI16, (T)IFDDA_SIN_PI8, (T)IFDDA_SIN_PI16, (T)0};
 #pragma unroll
         for (int k = 0; k < 16; k++) {
             // w32^k = cos(k pi/16) + i DIR sin(k pi/16)
+            if (k == 8) {
+                v[k] = cadd_i<DIR>(e[k], o[k]);
+                v[k + 16] = cadd_i<-DIR>(e[k], o[k]);
+                continue;
+            }
             const T c = k <= 8 ? cs[k] : -cs[16 - k];
             const T sn = k <= 8 ? cs[8 - k] : cs[k - 8];
-            const C w = mk(c, DIR > 0 ? sn : -sn);
-            const C t = k == 0 ? o[0] : cmul(o[k], w);
+            const C t = k == 0 ? o[0] : cmulk(o[k], c, DIR > 0 ? sn : -sn);
             v[k] = cadd(e[k], t);
             v[k + 16] = csub(e[k], t);
         }
     }
+    __device__ __forceinline__ static void run(C* v) { go<false>(v); }
+    __device__ __forceinline__ static void run_half(C* v) { go<true>(v); }
 };
-
-// 12 points as 4 x 3: DFT3 over the stride-4 subsequences, the twiddles
-// w12^(n2 k1), then DFT4 across them; X[k1 + 3 k2]
-template <int DIR, class C> struct Dft<12, DIR, C> {
-    __device__ __forceinline__ static void run(C* v);
-};
-
-template <int DIR, class C> struct Dft<3, DIR, C> {
-    __device__ __forceinline__ static void run(C* v) {
-        using T = decltype(C().x);
-        C t1 = cadd(v[1], v[2]);
-        C t2 = csub(v[0], cscale(t1, (T)0.5));
-        C t3 = cmul_i<DIR>(cscale(csub(v[1], v[2]), (T)IFDDA_SQRT3_2));
-        v[0] = cadd(v[0], t1);
-        v[1] = cadd(t2, t3);
-        v[2] = csub(t2, t3);
-    }
-};
-
-template <int DIR, class C> struct Dft<5, DIR, C> {
-    __device__ __forceinline__ static void run(C* v) {
-        using T = decltype(C().x);
-        const T c1 = (T)IFDDA_C1_5, c2 = (T)IFDDA_C2_5, s1 = (T)IFDDA_S1_5, s2 = (T)IFDDA_S2_5;
-        C t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
-        C t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-        C a1 = cadd(v[0], cadd(cscale(t1, c1), cscale(t2, c2)));
-        C a2 = cadd(v[0], cadd(cscale(t1, c2), cscale(t2, c1)));
-        C b1 = cmul_i<DIR>(cadd(cscale(t3, s1), cscale(t4, s2)));
-        C b2 = cmul_i<DIR>(csub(cscale(t3, s2), cscale(t4, s1)));
-        v[0] = cadd(v[0], cadd(t1, t2));
-        v[1] = cadd(a1, b1);
-        v[4] = csub(a1, b1);
-        v[2] = cadd(a2, b2);
-        v[3] = csub(a2, b2);
-    }
-};
-
-template <int DIR, class C> __device__ __forceinline__ void Dft<12, DIR, C>::run(C* v) {
-    using T = decltype(C().x);
-    C a[4][3];
-#pragma unroll
-    for (int n2 = 0; n2 < 4; n2++) {
-        C t[3] = {v[n2], v[4 + n2], v[8 + n2]};
-        Dft<3, DIR, C>::run(t);
-#pragma unroll
-        for (int k1 = 0; k1 < 3; k1++) a[n2][k1] = t[k1];
-    }
-    // w12^1 = (sqrt3/2, DIR/2), w12^2 = (1/2, DIR sqrt3/2), w12^4 = (-1/2, DIR sqrt3/2)
-    const T h = (T)0.5, r3 = (T)IFDDA_SQRT3_2;
-    const C w1 = mk(r3, DIR > 0 ? h : -h), w2 = mk(h, DIR > 0 ? r3 : -r3), w4 = mk(-h, DIR > 0 ? r3 : -r3);
-    a[1][1] = cmul(a[1][1], w1);
-    a[1][2] = cmul(a[1][2], w2);
-    a[2][1] = cmul(a[2][1], w2);
-    a[2][2] = cmul(a[2][2], w4);
-    a[3][1] = cmul_i<DIR>(a[3][1]);  // w12^3
-    a[3][2] = cscale(a[3][2], (T)-1);  // w12^6
-#pragma unroll
-    for (int k1 = 0; k1 < 3; k1++) {
-        C t[4] = {a[0][k1], a[1][k1], a[2][k1], a[3][k1]};
-        Dft<4, DIR, C>::run(t);
-#pragma unroll
-        for (int k2 = 0; k2 < 4; k2++) v[k1 + 3 * k2] = t[k2];
-    }
-}
 
 // Source / destination that is the shared-memory tile itself.
 struct SmemIO {
@@ -317,14 +464,15 @@ struct SmemIO {
 // PADSH > 0 inserts one padding word every 2^PADSH points, so the strided
 // writes of a radix-R pass (points j*R + r of consecutive j) spread over the
 // shared-memory banks.
-template <int PS_, int BS_, bool BFAST_, int PADSH_ = 0> struct Layout {
-    static constexpr int PS = PS_, BS = BS_, PADSH = PADSH_;
+// PADOFF shifts where the padding words fall.
+template <int PS_, int BS_, bool BFAST_, int PADSH_ = 0, int PADOFF_ = 0> struct Layout {
+    static constexpr int PS = PS_, BS = BS_, PADSH = PADSH_, PADOFF = PADOFF_;
     static constexpr bool BFAST = BFAST_;
     // padded position of point p
-    __host__ __device__ static constexpr int pidx(int p) { return PADSH ? p + (p >> PADSH) : p; }
+    __host__ __device__ static constexpr int pidx(int p) { return PADSH ? p + ((p + PADOFF) >> PADSH) : p; }
     __device__ __forceinline__ static int addr(int p, int b) { return pidx(p) * PS + b * BS; }
     // points spanned by a line of length L (padding included)
-    static constexpr int span(int L) { return PADSH ? L + (L >> PADSH) : L; }
+    static constexpr int span(int L) { return PADSH ? L + ((L + PADOFF) >> PADSH) : L; }
 };
 
 // True when the padded positions of a butterfly's points j + r NJ (j < NJ,
@@ -348,7 +496,9 @@ template <class Lay> constexpr bool write_split(int NJ, int Ns, int R) {
 
 // One Stockham pass.  tw[j] = exp(+2 pi i j / L) in shared memory.
 template <class C, int L, int R, int Ns, int NB, int NT, int DIR, class Lay, class Src, class Dst>
-__device__ __forceinline__ void stockham_pass(C* sm, const C* tw, const Src& src, const Dst& dst) {
+__device__ __forceinline__ void stockham_pass(C* sm, const typename elem_traits<C>::W* tw, const Src& src,
+                                              const Dst& dst, const int tid) {
+    using W = typename elem_traits<C>::W;
     constexpr int NJ = L / R;
     constexpr int NBF = NB * NJ;
     constexpr int PER = (NBF + NT - 1) / NT;
@@ -356,75 +506,98 @@ __device__ __forceinline__ void stockham_pass(C* sm, const C* tw, const Src& src
     constexpr bool FIRST = Ns == 1, LAST = Ns * R == L;
     constexpr bool GIN = FIRST && Src::GLOBAL, GOUT = LAST && Dst::GLOBAL;
     constexpr bool RSPLIT = read_split<Lay>(NJ, R), WSPLIT = write_split<Lay>(NJ, Ns, R);
-    C v[PER][R];
+    // one butterfly: inputs, twiddles, transform
+    const auto read = [&](C(&v)[R], int u) {
+        const int b = Lay::BFAST ? u % NB : u / NJ;
+        const int j = Lay::BFAST ? u / NB : u % NJ;
 #pragma unroll
-    for (int q = 0; q < PER; q++) {
-        const int u = threadIdx.x + q * NT;
-        if (PER * NT == NBF || u < NBF) {
-            const int b = Lay::BFAST ? u % NB : u / NJ;
-            const int j = Lay::BFAST ? u / NB : u % NJ;
-#pragma unroll
-            for (int r = 0; r < R; r++) {
-                const int p = j + r * NJ;
-                if (GIN) {
-                    // zero upper half: for an even radix p >= L/2 exactly when r >= R/2
-                    const bool zero = Src::HALF && (R % 2 == 0 ? 2 * r >= R : 2 * p >= L);
-                    v[q][r] = zero ? mk(decltype(C().x)(0), decltype(C().x)(0)) : src.template load<C>(b, p);
-                } else if constexpr (RSPLIT) {
-                    v[q][r] = sm[Lay::addr(j, b) + Lay::pidx(r * NJ) * Lay::PS];
-                } else {
-                    v[q][r] = sm[Lay::addr(p, b)];
-                }
+        for (int r = 0; r < R; r++) {
+            const int p = j + r * NJ;
+            if (GIN) {
+                // zero upper half: for an even radix p >= L/2 exactly when r >= R/2
+                const bool zero = Src::HALF && (R % 2 == 0 ? 2 * r >= R : 2 * p >= L);
+                v[r] = zero ? czero<C>() : src.template load<C>(b, p);
+            } else if constexpr (RSPLIT) {
+                v[r] = sm[Lay::addr(j, b) + Lay::pidx(r * NJ) * Lay::PS];
+            } else {
+                v[r] = sm[Lay::addr(p, b)];
             }
-            if (Ns > 1) {
-                const int k = j % Ns;
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    C w = tw[k * r * TSTEP];
-                    if (DIR < 0) w = cconj(w);
-                    v[q][r] = cmul(v[q][r], w);
-                }
-            }
-            Dft<R, DIR, C>::run(v[q]);
         }
-    }
-    if (!GIN) __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-        const int u = threadIdx.x + q * NT;
-        if (PER * NT == NBF || u < NBF) {
-            const int b = Lay::BFAST ? u % NB : u / NJ;
-            const int j = Lay::BFAST ? u / NB : u % NJ;
+        if (Ns > 1) {
             const int k = j % Ns;
-            const int d = (j / Ns) * Ns * R + k;
 #pragma unroll
-            for (int r = 0; r < R; r++) {
-                const int o = d + r * Ns;
-                if (GOUT) {
-                    // last pass: o = j + r L/R; for an even radix o < L/2 exactly when r < R/2
-                    const bool keep = !Dst::HALF || (R % 2 == 0 ? 2 * r < R : 2 * o < L);
-                    if (keep) dst.template store<C>(b, o, v[q][r]);
-                } else if constexpr (WSPLIT) {
-                    sm[Lay::addr(d, b) + Lay::pidx(r * Ns) * Lay::PS] = v[q][r];
-                } else {
-                    sm[Lay::addr(o, b)] = v[q][r];
-                }
+            for (int r = 1; r < R; r++) {
+                W w = tw[k * r * TSTEP];
+                if (DIR < 0) w = cconj(w);
+                v[r] = cmul(v[r], w);
             }
         }
+        if constexpr (GIN && Src::HALF && R % 2 == 0) Dft<R, DIR, C>::run_half(v);
+        else Dft<R, DIR, C>::run(v);
+    };
+    const auto write = [&](const C(&v)[R], int u) {
+        const int b = Lay::BFAST ? u % NB : u / NJ;
+        const int j = Lay::BFAST ? u / NB : u % NJ;
+        const int k = j % Ns;
+        const int d = (j / Ns) * Ns * R + k;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int o = d + r * Ns;
+            if (GOUT) {
+                // last pass: o = j + r L/R; for an even radix o < L/2 exactly when r < R/2
+                const bool keep = !Dst::HALF || (R % 2 == 0 ? 2 * r < R : 2 * o < L);
+                if (keep) dst.template store<C>(b, o, v[r]);
+            } else if constexpr (WSPLIT) {
+                sm[Lay::addr(d, b) + Lay::pidx(r * Ns) * Lay::PS] = v[r];
+            } else {
+                sm[Lay::addr(o, b)] = v[r];
+            }
+        }
+    };
+    if constexpr (GIN || GOUT) {
+        // the tile is only written or only read: one butterfly after the other, no barrier between
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int u = tid + q * NT;
+            if (PER * NT == NBF || u < NBF) {
+                C v[R];
+                read(v, u);
+                write(v, u);
+            }
+        }
+    } else {
+        C v[PER][R];
+#pragma unroll
+        for (int q = 0; q < PER; q++)
+            if (PER * NT == NBF || tid + q * NT < NBF) read(v[q], tid + q * NT);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; q++)
+            if (PER * NT == NBF || tid + q * NT < NBF) write(v[q], tid + q * NT);
     }
     if (!GOUT) __syncthreads();
 }
 
 // Passes q in [q, Q1) of the plan (reversed when REV); Ns is the product of
-// the radices of the passes before q.
+// the radices of the passes before q.  tid is the thread's index; a caller
+// that loops passes it through loop_tid() below, so that the compiler does not
+// keep every twiddle and tile address of the loop body in registers.
 template <class C, int L, int NB, int NT, int DIR, class Lay, bool REV, int Q1, int q, int Ns, class Src, class Dst,
           int PLAN = 0>
-__device__ __forceinline__ void stockham_range(C* sm, const C* tw, const Src& src, const Dst& dst) {
+__device__ __forceinline__ void stockham_range(C* sm, const typename elem_traits<C>::W* tw, const Src& src,
+                                               const Dst& dst, const int tid = threadIdx.x) {
     if constexpr (q < Q1) {
         constexpr int R = plan_radix_dir(L, q, REV, PLAN);
-        stockham_pass<C, L, R, Ns, NB, NT, DIR, Lay, Src, Dst>(sm, tw, src, dst);
-        stockham_range<C, L, NB, NT, DIR, Lay, REV, Q1, q + 1, Ns * R, Src, Dst, PLAN>(sm, tw, src, dst);
+        stockham_pass<C, L, R, Ns, NB, NT, DIR, Lay, Src, Dst>(sm, tw, src, dst, tid);
+        stockham_range<C, L, NB, NT, DIR, Lay, REV, Q1, q + 1, Ns * R, Src, Dst, PLAN>(sm, tw, src, dst, tid);
     }
+}
+
+// threadIdx.x as a value the compiler takes to change from iteration to iteration
+__device__ __forceinline__ int loop_tid() {
+    int t = threadIdx.x;
+    asm volatile("" : "+r"(t));
+    return t;
 }
 
 // Transform NB lines.  When the source is shared memory the caller must have
@@ -432,10 +605,11 @@ __device__ __forceinline__ void stockham_range(C* sm, const C* tw, const Src& sr
 // result may be read right after the call (the last pass ends in a barrier).
 // The twiddle table must be resident before the second pass (the first pass
 // uses none), so a caller may start filling it together with the first pass.
-template <class C, int L, int NB, int NT, int DIR, class Lay, class Src = SmemIO, class Dst = SmemIO>
-__device__ __forceinline__ void fft_tile(C* sm, const C* tw, const Src& src = Src(), const Dst& dst = Dst()) {
+template <class C, int L, int NB, int NT, int DIR, class Lay, class Src = SmemIO, class Dst = SmemIO, int PLAN = 0>
+__device__ __forceinline__ void fft_tile(C* sm, const typename elem_traits<C>::W* tw, const Src& src = Src(),
+                                         const Dst& dst = Dst()) {
     static_assert(smooth235(L), "FFT length must be a product of 2, 3 and 5");
-    stockham_range<C, L, NB, NT, DIR, Lay, false, plan_len(L), 0, 1, Src, Dst>(sm, tw, src, dst);
+    stockham_range<C, L, NB, NT, DIR, Lay, false, plan_len(L, PLAN), 0, 1, Src, Dst, PLAN>(sm, tw, src, dst);
 }
 
 // shared-memory to shared-memory transform with lines fastest (LS >= NB)

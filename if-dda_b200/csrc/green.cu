@@ -214,9 +214,8 @@ void green_export(const Green& G, double2* const out[6], cudaStream_t st) {
     std::vector<double2> h((size_t)6 * g.gc_comp);
     IFDDA_CUDA(cudaMemcpyAsync(h.data(), G.gc64.p, h.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
     IFDDA_CUDA(cudaStreamSynchronize(st));
-    const int W = g.nx + 1, H = g.ny + 1;
+    const int W = g.nx + 1, D = g.nz + 1;
     for (int c = 0; c < 6; c++) {
-        const double2* src = h.data() + (size_t)c * g.gc_comp;
         for (int kz = 0; kz < g.Z; kz++) {
             const int qz = kz <= g.nz ? kz : g.Z - kz;
             const int sz = kz <= g.nz ? 1 : parity(c, 2);
@@ -227,7 +226,7 @@ void green_export(const Green& G, double2* const out[6], cudaStream_t st) {
                     const int qx = ix <= g.nx ? ix : g.X - ix;
                     const int sx = ix <= g.nx ? 1 : parity(c, 0);
                     const double s = (double)(sx * sy * sz);
-                    const double2 v = src[((size_t)qz * H + qy) * W + qx];
+                    const double2 v = h[(((size_t)qy * W + qx) * 6 + c) * D + qz];
                     out[c][((size_t)kz * g.Y + jy) * g.X + ix] = make_double2(s * v.x, s * v.y);
                 }
             }

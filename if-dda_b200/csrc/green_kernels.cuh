@@ -7,7 +7,8 @@
 //        (calculgreenfft.f:25-69), FFT along x (sign +1), keep qx in [0, nx]
 //                                                          -> GA[c][nz+1][ny+1][nx+1]
 //   gy : FFT along y, keep qy in [0, ny]                   -> GB[c][nz+1][ny+1][nx+1]
-//   gz : FFT along z, keep qz in [0, nz]                   -> Gc64, Gc32
+//   gz : FFT along z, keep qz in [0, nz]                   -> Gc64, Gc32,
+//        Gc[ny+1][nx+1][c][nz+1] (z fastest)
 // Only the parity octant is kept: every component is even or odd along each
 // axis, so the rest of the spectrum is a mirror image (see matvec_kernels.cuh).
 // The same parity holds in real space, T_c(x, -y, z) = Py(c) T_c(x, y, z) and
@@ -39,7 +40,9 @@ template <int L> struct GreenTiles {
     static constexpr int NT = 256;
     static constexpr int LSX = (6 * TLX) | 1;
     static constexpr size_t smem_x = (size_t)L * S + (size_t)L * LSX * S;
-    static constexpr size_t smem_y = (size_t)L * S + (size_t)L * TLY * S;
+    // one column of padding: the z pass reads its lines point by point
+    static constexpr int LSY = TLY + 1;
+    static constexpr size_t smem_y = (size_t)L * S + (size_t)L * LSY * S;
 };
 
 // T_ab(r), the six independent components xx, xy, xz, yy, yz, zz
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_x(const GreenGeom g
 }
 
 // AXIS 1: GA[c][nz+1][ny+1][W] -> GB[c][nz+1][ny+1][W], rows y > ny read as
-// Py(c) times row Y - y;  AXIS 2: GB -> Gc[c][nz+1][ny+1][W], planes z > nz
+// Py(c) times row Y - y;  AXIS 2: GB -> Gc[ny+1][W][c][nz+1], planes z > nz
 // read as Pz(c) times plane Z - z
 template <int L, int AXIS>
 __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_yz(const GreenGeom g, const double2* __restrict__ src,
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_yz(const GreenGeom 
                                                                 const double2* __restrict__ tw_axis) {
     using C = double2;
     using TT = GreenTiles<L>;
-    constexpr int TL = TT::TLY, NT = TT::NT;
+    constexpr int TL = TT::TLY, LS = TT::LSY, NT = TT::NT;
     extern __shared__ __align__(16) unsigned char raw[];
     C* tw = reinterpret_cast<C*>(raw);
     C* sm = tw + L;
@@ -230,20 +233,26 @@ __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_yz(const GreenGeom 
             v = src[idx];
             if (p > half) v = make_double2(sgn * v.x, sgn * v.y);
         }
-        sm[e] = v;
+        sm[p * LS + il] = v;
     }
     __syncthreads();
-    tile_fft<C, L, TL, TL, NT, +1>(sm, tw);
-    for (int e = threadIdx.x; e < TL * keep; e += NT) {
-        const int p = e / TL, il = e - p * TL;
-        const int q = q0 + il;
-        if (q >= W) continue;
-        long idx;
-        if (AXIS == 1) idx = (((long)c * (g.nz + 1) + o) * (g.ny + 1) + p) * W + q;
-        else idx = (((long)c * (g.nz + 1) + p) * (g.ny + 1) + o) * W + q;
-        const C v = sm[e];
+    tile_fft<C, L, TL, LS, NT, +1>(sm, tw);
+    const auto put = [&](int p, int il, long idx) {
+        const C v = sm[p * LS + il];
         dst64[idx] = v;
         if (AXIS == 2 && dst32) dst32[idx] = make_float2((float)v.x, (float)v.y);
+    };
+    if constexpr (AXIS == 1) {
+        for (int e = threadIdx.x; e < TL * keep; e += NT) {
+            const int p = e / TL, il = e - p * TL;
+            if (q0 + il < W) put(p, il, (((long)c * (g.nz + 1) + o) * (g.ny + 1) + p) * W + q0 + il);
+        }
+    } else {  // a warp writes one line: z is contiguous
+        for (int il = threadIdx.x / 32; il < TL; il += NT / 32) {
+            if (q0 + il >= W) break;
+            const long line = (((long)o * W + q0 + il) * 6 + c) * (g.nz + 1);
+            for (int p = threadIdx.x & 31; p < keep; p += 32) put(p, il, line + p);
+        }
     }
 }
 

@@ -19,13 +19,24 @@
 // registers of the last one (the cropped half is never written); shared memory
 // holds the tile between the inner FFT passes only.
 //
+// Order along X in B1 and B2: the frequencies qx = t and X - t lie side by
+// side, at 2 t and 2 t + 1 (t = 0: qx = 0 and nx, which are their own
+// mirrors).  Both see the same spectrum values up to the sign of xy and xz,
+// which the x passes take out by storing component x of the mirrored one
+// negated (S G S v with S = diag(-1, 1, 1)), so the y and z passes read one
+// column of G~ for two columns of data.  In FP64 the two are neighbouring
+// 16-byte elements; in FP32 they form one 16-byte element (cpair: both real
+// parts, both imaginary parts), on which sums take one packed instruction
+// for two values.  The x passes' butterflies j and X/R - j hold the
+// frequencies t and X - t together, so a thread that does both writes or
+// reads whole pairs.
+//
 // The compressed spectrum: G(r) on the circulant grid is even (xx,yy,zz) or odd
 // (xy in x,y; xz in x,z; yz in y,z) under q -> (L - q) mod L along each axis
 // (zero planes at nx,ny,nz, cdmlib/calculgreenfft.f:29-35), so its DFT has the
-// same parity and only q in [0, L/2] per axis is stored:
-//   Gc[c6][qz][qy][qx], dims (nz+1, ny+1, nx+1), c6 = xx,xy,xz,yy,yz,zz.
-// zconv treats the mirror rows qy and Y-qy in one block, so each compressed
-// value read serves both.
+// same parity and only q in [0, L/2] per axis is stored, z fastest so that
+// what a column of zconv needs is contiguous:
+//   Gc[qy][qx][c6][qz], dims (ny+1, nx+1, 6, nz+1), c6 = xx,xy,xz,yy,yz,zz.
 #pragma once
 #include "fft_tile.cuh"
 #include "reduce.cuh"
@@ -38,7 +49,7 @@ struct MvGeom {
     long N;             // nx*ny*nz
     long b1_rhs;        // elements of B1 per right-hand side: 3*nz*ny*X
     long b2_rhs;        // elements of B2 per right-hand side: 3*nz*Y*X
-    long gc_comp;       // elements of one compressed G~ component
+    long gc_comp;       // octant sites (nx+1)(ny+1)(nz+1): elements of one compressed G~ component
 };
 
 // polarisability modes
@@ -76,28 +87,37 @@ template <class T> struct MvArgs {
 };
 
 // Tile shapes: lines per block, threads per block and the register cap of
-// each pass.  The rules come from a sweep of every pass over tile widths,
-// thread counts and register caps on B200 at the 128^3 (FP32, FP64),
-// 192x192x128 (8 right-hand sides) and 384^3 grids:
-//  * x passes: latency-bound at small grids (every shape within 5%); a cap of
-//    80 (FP32) / 96 (FP64) registers helps the larger grids;
-//  * y passes: 16 columns per block (64 contiguous bytes per row in FP32) at
-//    every length, about 30% faster than narrower tiles at 192 and 384;
-//  * zconv: as many columns as fit in ~80 KB (FP32) / ~160 KB (FP64) of
-//    shared memory, so that two blocks (FP32) share an SM, and a register
-//    cap near 72 (FP32) / 168 (FP64) to keep more blocks resident.
+// each pass, with what they measured on B200.
+//  * x passes: about 16 KB of shared memory (8 KB below length 64, where a
+//    small lattice would otherwise leave SMs without a block).  FP32 keeps to 80
+//    registers: at 96 the 1024 blocks of a 64^3 grid no longer fit the SMs at
+//    once, and the solver's passes took 24.9 instead of 18.5 us;
+//  * y passes: 8 columns of 16 bytes, 16 (V = 1);
+//  * zconv: 8 columns of 16 bytes, rows of 128 bytes.  4 columns (V = 1 below
+//    160) and 2 give more and smaller blocks, but their narrower rows cost more
+//    than that: FP64 at 64^3 43.5, 47.5 and 65 us, FP32 27.9, 29.5 and 40.5 us.
+//    From 160 on two passes need 150 to 250 registers a thread, which leaves 6
+//    to 12 warps per SM; there V = 1 takes three passes of small radices at 80
+//    registers and reads the spectrum where it uses it (L2), so that 24 warps
+//    fit: FP32 at 192^3 1.21 -> 0.89 ms.  Below, where two passes leave 12 warps
+//    or more, three were slower (FP64 at 64^3 57.9 against 45.2 us: the extra
+//    round trip through shared memory).
+// The variants are compiled for lengths of 64 and more; the tile chooser
+// (tune_tiles) times both on the caller's grid and keeps one per grid.  The
+// two agree to rounding.
 //
-// Variant V = 1 (compiled for lengths of 64 and more, where the grid is large
-// enough for the choice to matter) halves the zconv and y tiles; the tile
-// chooser (tune_tiles) times both on the caller's grid and keeps one per
-// grid.  The two agree to rounding (the compiler may contract multiply-adds
-// differently in the two instances).
+// Tried without gain and left out: B2 stored in column tiles (z rows no longer
+// a power of two apart), a persistent zconv that copies the next row's input
+// under the current one (FP64 at 64^3 49 against 43.5 us), right-hand sides and
+// column slabs run through the passes in groups that fit L2.
 constexpr int tile_variants(int L) { return L >= 64 ? 2 : 1; }
 template <class T, int L, int V = 0> struct MvTiles {
+    using E = typename yz_elem<T>::type;
     static constexpr int S = (int)sizeof(cplx<T>);
-    static constexpr int SMEM_X = 16384;
+    static constexpr int SE = (int)sizeof(E);
+    static constexpr int SMEM_X = L >= 64 ? 16384 : 8192;
     static constexpr int TLX = clamp_pow2(SMEM_X / (3 * (L + 1) * S), 1, 16);
-    static constexpr int TLY = V ? 8 : 16;
+    static constexpr int TLY = V ? 16 : 8;
     static constexpr int NBX = 3 * TLX, NBY = TLY;
     // x tile: points contiguous with one pad word every 16, line pitch = 8 (mod 16)
     static constexpr int lpitch() {
@@ -106,73 +126,87 @@ template <class T, int L, int V = 0> struct MvTiles {
         return p;
     }
     static constexpr int LP = lpitch();
-    // one butterfly of the widest radix per thread
-    static constexpr int nthreads(int nb, int policy = 0) {
-        int t = nb * L / max_radix(L, policy);
+    static constexpr int round32(int t, int hi) {
         t = (t + 31) / 32 * 32;
-        return t < 64 ? 64 : (t > 512 ? 512 : t);
+        return t > hi ? hi : t;
     }
-    // blocks per SM asked of the compiler so that it keeps to about cap registers
+    // blocks per SM asked of the compiler so that it keeps to about cap
+    // registers: a quarter of the SM holds 512 registers for each lane of its warps
     static constexpr int minblocks(int nt, int cap) {
-        int m = 65536 / (nt * cap);
+        int m = 4 * (512 / cap) / (nt / 32);
         if (m * nt > 2048) m = 2048 / nt;
         return m < 1 ? 1 : (m > 32 ? 32 : m);
     }
-    // z tile: shared memory of TL columns of mr mirror rows (twiddles, data
-    // tile with one pad point every 16, the block's slice of the compressed
-    // spectrum)
-    static constexpr size_t zbytes(int tl, int mr = 2) {
-        return (size_t)L * S + (size_t)(L + (L >> 4)) * 3 * mr * tl * S + (size_t)6 * (L / 2 + 1) * tl * S;
+    // x passes: radix of the last forward (first inverse) pass, its
+    // butterflies per line and pairs of them (j, NJ - j)
+    static constexpr int NPX = plan_len(L, PLAN_X);
+    static constexpr int RX = plan_radix(L, NPX - 1, PLAN_X), NJX = L / RX, NJP = (NJX + 1) / 2;
+    static constexpr int NTX = round32(NPX > 2 || NBX * NJP > NBX * (L / plan_radix(L, 0, PLAN_X))
+                                           ? NBX * NJP : NBX * (L / plan_radix(L, 0, PLAN_X)), 512);
+    // y passes: one butterfly of the first radix per thread
+    static constexpr int RY = plan_radix(L, 0, PLAN_Y);
+    static constexpr int NTY = round32(NBY * (L / RY), 512);
+    // zconv: first radix, middle radix (the last of the plan), groups of the
+    // middle per column
+    // V = 1 from length 160 on: three small radices, and the spectrum read
+    // from L2 where it is used instead of through shared memory
+    static constexpr bool ZSMALL = V == 1 && L >= 160;
+    static constexpr int PZ = ZSMALL ? PLAN_Z3 : PLAN_Z;
+    static constexpr int NPZ = plan_len(L, PZ);
+    static constexpr int RZ = plan_radix(L, 0, PZ), RK = plan_radix(L, NPZ - 1, PZ), NJZ = L / RK;
+    // Tiles of 8 columns need no padding: 8 lanes of 16 bytes fill the banks.
+    // With fewer, the butterflies j, j + 1 of the middle (RK a power of two)
+    // must lie an odd number of points apart.
+    static constexpr int log2i(int v) { return v <= 1 ? 0 : 1 + log2i(v / 2); }
+    static constexpr bool RKP2 = RK == 2 || RK == 4 || RK == 8;
+    static constexpr int zpadsh(int tl) { return tl >= 8 ? 0 : (RKP2 ? log2i(2 * RK) : RK == 12 ? 2 : 4); }
+    static constexpr int zpadoff(int tl) { return tl >= 8 || !RKP2 ? 0 : RK; }
+    static constexpr int zspan(int tl) { return zpadsh(tl) ? L + ((L + zpadoff(tl)) >> zpadsh(tl)) : L; }
+    // G~ slice: columns of the tile (pairs share one) and one for qx = nx;
+    // pitch of a column in W elements, a multiple of 16 bytes, chosen so that
+    // neighbouring columns fall into different banks
+    static constexpr int NQ = L / 2 + 1;
+    static constexpr int gcols(int tl) { return S == 8 ? tl : tl / 2; }
+    static constexpr int gpitch() {
+        int g = 6 * NQ;
+        if (S == 8) {
+            while (g % 8 != 4) g++;
+        } else {
+            while (g % 8 != 2 && g % 8 != 6) g++;
+        }
+        return g;
     }
-    // zconv's FFT plan in FP32: two passes (a 32- or 16-point first pass)
-    // where that saves a pass over the usual plan (lengths 96, 160, 192, 256,
-    // 384), at about 120 registers a thread; FP64 keeps the usual plan (its
-    // 12-point middle for three components would not fit the registers)
-    static constexpr int ZP = (S == 8 && plan_len(L, 1) > 0 && plan_len(L, 1) < plan_len(L, 0)) ? 1 : 0;
-    // With the two-pass plan the tile is wider (up to ~120 KB, 32-byte rows
-    // at 384), one block per SM.  Variant 1 takes one of the two mirror rows
-    // per block (MRZ = 1) and as many columns as fit (up to ~160 KB with the
-    // two-pass plan, 64-byte rows at 384; up to 112 KB otherwise, so that two
-    // blocks share an SM in FP64 too): wider rows, whose DRAM accesses are
-    // less scattered, the spectrum slice then read by the two blocks of a row
-    // pair back to back (L2 serves the second).  The tile chooser times the
-    // two.
-    static constexpr int MRZ = V ? 1 : 2;
+    static constexpr int GST = gpitch();
+    static constexpr size_t zbytes(int tl) {
+        return (size_t)L * S + (size_t)zspan(tl) * 3 * tl * SE + (ZSMALL ? 0 : (size_t)(gcols(tl) + 1) * GST * S);
+    }
     static constexpr int ztile() {
-        const size_t budget = MRZ == 1 ? (size_t)(ZP ? 160 : 112) * 1024 : (size_t)(ZP ? 120 : 80) * 1024 * (S / 8);
-        int tl = 16;
-        while (tl > 1 && zbytes(tl, MRZ) > budget) tl /= 2;
+        int tl = V == 1 && !ZSMALL ? 4 : 8;
+        while (tl > 2 && zbytes(tl) > 112 * 1024) tl /= 2;
         return tl;
     }
-    static constexpr int TLZ = ztile(), NBZ = 3 * MRZ * TLZ;
+    static constexpr int TLZ = ztile(), NBZ = 3 * TLZ, TCZ = gcols(TLZ);
+    static_assert(TLZ >= 2, "a zconv tile holds whole pairs");
+    static constexpr int NTZ = ZSMALL ? round32(TLZ * NJZ, 512) : round32(NBZ * (L / RZ) > TLZ * NJZ ? NBZ * (L / RZ) : TLZ * NJZ, 512);
     // L2 prefetch size of the column reads of zconv and the y passes (rows of
-    // TLZ or TLY columns, 32 to 128 bytes, that neighbouring blocks read at
-    // the same time): 256-byte DRAM bursts, 4-5% faster at 192^2 x 128 and 384^3
+    // 32 to 256 bytes that neighbouring blocks read at the same time)
     static constexpr int ZPF = 256;
-    // y tile: odd point stride; z tile: point stride NBZ with one pad point every 16
-    static constexpr int PSY = NBY + 1, PSZ = NBZ;
     using LayX = Layout<1, LP, false, 4>;
-    using LayY = Layout<PSY, 1, true>;
-    using LayZ = Layout<PSZ, 1, true, 4>;
-    static constexpr int NTX = nthreads(NBX), NTY = nthreads(NBY), NTZ = nthreads(NBZ, ZP);
-    static constexpr int MINBX = minblocks(NTX, S == 8 ? 80 : 96);
-    static constexpr int MINBY = minblocks(NTY, S == 8 ? 80 : 112);
-    static constexpr int MINBZ = minblocks(NTZ, S == 8 ? (ZP ? 128 : 72) : 168);
+    using LayY = Layout<NBY, 1, true>;
+    using LayZ = Layout<NBZ, 1, true, zpadsh(TLZ), zpadoff(TLZ)>;
+    static constexpr int MINBX = minblocks(NTX, S == 8 ? 80 : (RX > 8 ? 128 : 102));
+    static constexpr int MINBY = minblocks(NTY, RY == 32 ? 168 : 128);
+    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : 128));
     static constexpr size_t smem_x = (size_t)L * S + (size_t)NBX * LP * S;
-    static constexpr size_t smem_y = (size_t)L * S + (size_t)L * PSY * S;
-    static constexpr size_t smem_z = (size_t)L * S + (size_t)LayZ::span(L) * PSZ * S +
-                                     (size_t)6 * (L / 2 + 1) * TLZ * S;
-    static_assert(zbytes(TLZ, MRZ) == smem_z, "z tile size rule and layout disagree");
+    static constexpr size_t smem_y = (size_t)L * S + (size_t)L * NBY * SE;
+    static constexpr size_t smem_z = zbytes(TLZ);
+    static_assert(smem_z <= 227 * 1024 && smem_y <= 227 * 1024 && smem_x <= 227 * 1024, "tile above the SM's shared memory");
 };
 
-// asynchronous global -> shared copy of one complex element (8 or 16 bytes);
-// PF = 256 asks L2 to fetch the 256 bytes around it from DRAM
-template <int PF = 0, class C> __device__ __forceinline__ void cp_async_elem(C* dst_smem, const C* src) {
+// asynchronous global -> shared copy of 16 bytes
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-    if constexpr (PF == 256)
-        asm volatile("cp.async.ca.shared.global.L2::256B [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"((int)sizeof(C)));
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"((int)sizeof(C)));
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;\n" ::"r"(d), "l"(src));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
@@ -230,29 +264,134 @@ template <class T, bool TAB, class Pre> struct FwdXLoad {
     }
 };
 
-// B1 rows of one x-pass tile: line b = c * TL + jl is row ((c * nz + k) * ny + j0 + jl)
-template <class T, int L, int TL> struct B1RowIO {
-    static constexpr bool GLOBAL = true, HALF = false;
-    cplx<T>* base;  // row (c = 0, k, j0) of this right-hand side
-    int nl, cstride;  // valid rows, elements between components (nz ny L)
-    template <class C> __device__ __forceinline__ int at(int b, int p) const {
+// Frequencies of a pair of butterflies (jA = jp, jB) of radix R on a line of
+// length L = R NJ: butterfly j holds j + r NJ, r < R.  For jp > 0, jB = NJ - jp
+// holds the mirrors: r of one is R - 1 - r of the other.  jp = 0 and (NJ even)
+// jB = NJ / 2 hold their own: r and R - r (0 and R / 2 pair up as t = 0), and
+// r and R - 1 - r.  NJ odd: jp = 0 has no jB.
+template <int NJ> __device__ __forceinline__ int pair_jb(int jp) { return jp == 0 ? NJ / 2 : NJ - jp; }
+
+// one element pair t of a B1 row: first = frequency t, second = X - t
+__device__ __forceinline__ void pair_store(float2* row, int t, float2 f, float2 s) {
+    reinterpret_cast<cpair*>(row)[t] = cpair{make_float2(f.x, s.x), make_float2(f.y, s.y)};
+}
+__device__ __forceinline__ void pair_store(double2* row, int t, double2 f, double2 s) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(row + 2 * t), "d"(f.x), "d"(f.y), "d"(s.x), "d"(s.y)
+                 : "memory");
+}
+__device__ __forceinline__ void pair_load(const float2* row, int t, float2& f, float2& s) {
+    const cpair v = reinterpret_cast<const cpair*>(row)[t];
+    f = make_float2(v.re.x, v.im.x);
+    s = make_float2(v.re.y, v.im.y);
+}
+__device__ __forceinline__ void pair_load(const double2* row, int t, double2& f, double2& s) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(f.x), "=d"(f.y), "=d"(s.x), "=d"(s.y)
+                 : "l"(row + 2 * t)
+                 : "memory");
+}
+
+// Last forward pass of an x tile: smem (or, for a one-pass plan, src) -> B1
+// pairs.  base: row (c = 0, k, j0); nl valid rows; cstride: elements between
+// components.
+template <class C, int L, class TT, class Src>
+__device__ __forceinline__ void x_store_pairs(const C* sm, const C* tw, const Src& src, C* base, int nl, int cstride) {
+    constexpr int R = TT::RX, NJ = TT::NJX, NJP = TT::NJP, NT = TT::NTX, TL = TT::TLX;
+    using Lay = typename TT::LayX;
+    constexpr int ITEMS = TT::NBX * NJP, PER = (ITEMS + NT - 1) / NT;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        const int u = threadIdx.x + q * NT;
+        if (!(PER * NT == ITEMS || u < ITEMS)) continue;
+        const int b = u / NJP, jp = u % NJP;
         const int c = b / TL, jl = b - c * TL;
-        return jl < nl ? c * cstride + jl * L + p : -1;
+        if (jl >= nl) continue;
+        const int jb = pair_jb<NJ>(jp);
+        const bool self = jp == 0;
+        C A[R], B[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if constexpr (TT::NPX == 1) {
+                A[r] = 2 * r >= R ? czero<C>() : src.template load<C>(b, r);
+                B[r] = czero<C>();
+            } else {
+                A[r] = sm[Lay::addr(jp + r * NJ, b)];
+                B[r] = sm[Lay::addr(jb + r * NJ, b)];
+                if (r > 0) {
+                    A[r] = cmul(A[r], tw[jp * r]);
+                    B[r] = cmul(B[r], tw[jb * r]);
+                }
+            }
+        }
+        Dft<R, +1, C>::run(A);
+        Dft<R, +1, C>::run(B);
+        C* row = base + c * cstride + jl * L;
+        const typename elem_traits<C>::T sx = c == 0 ? -1 : 1;
+#pragma unroll
+        for (int r = 0; r < R / 2; r++) {
+            const C own = r == 0 ? A[R / 2] : cscale(A[(R - r) % R], sx);  // t = 0 keeps its sign
+            const C mir = cscale(B[R - 1 - r], sx);
+            pair_store(row, jp + r * NJ, A[r], self ? own : mir);
+        }
+        if (NJ % 2 == 0 || !self) {
+#pragma unroll
+            for (int r = 0; r < R / 2; r++)
+                pair_store(row, jb + r * NJ, B[r], cscale(self ? B[R - 1 - r] : A[R - 1 - r], sx));
+        }
     }
-    template <class C> __device__ __forceinline__ void store(int b, int p, C v) const {
-        const int o = at<C>(b, p);
-        if (o >= 0) base[o] = v;
+}
+
+// First inverse pass of an x tile: B1 pairs -> smem (or, for a one-pass plan, dst)
+template <class C, int L, class TT, class Dst>
+__device__ __forceinline__ void x_load_pairs(C* sm, const Dst& dst, const C* base, int nl, int cstride) {
+    constexpr int R = TT::RX, NJ = TT::NJX, NJP = TT::NJP, NT = TT::NTX, TL = TT::TLX;
+    using Lay = typename TT::LayX;
+    constexpr int ITEMS = TT::NBX * NJP, PER = (ITEMS + NT - 1) / NT;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        const int u = threadIdx.x + q * NT;
+        if (!(PER * NT == ITEMS || u < ITEMS)) continue;
+        const int b = u / NJP, jp = u % NJP;
+        const int c = b / TL, jl = b - c * TL;
+        const int jb = pair_jb<NJ>(jp);
+        const bool self = jp == 0, has_b = NJ % 2 == 0 || !self;
+        const typename elem_traits<C>::T sx = c == 0 ? -1 : 1;
+        C A[R], B[R], sa[R / 2], sb[R / 2];
+        const C* row = base + c * cstride + jl * L;
+#pragma unroll
+        for (int r = 0; r < R / 2; r++) {
+            A[r] = B[r] = sa[r] = sb[r] = czero<C>();
+            if (jl < nl) {
+                pair_load(row, jp + r * NJ, A[r], sa[r]);
+                if (has_b) pair_load(row, jb + r * NJ, B[r], sb[r]);
+            }
+        }
+#pragma unroll
+        for (int r = R / 2; r < R; r++) {
+            const C own = r == R / 2 ? sa[0] : cscale(sa[R - r], sx);
+            const C mir = cscale(sb[R - 1 - r], sx);
+            A[r] = self ? own : mir;
+            B[r] = cscale(self ? sb[R - 1 - r] : sa[R - 1 - r], sx);
+        }
+        Dft<R, -1, C>::run(A);
+        Dft<R, -1, C>::run(B);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            if constexpr (TT::NPX == 1) {
+                if (2 * r < R) dst.template store<C>(b, r, A[r]);
+            } else {
+                sm[Lay::addr(jp * R + r, b)] = A[r];
+                if (has_b) sm[Lay::addr(jb * R + r, b)] = B[r];
+            }
+        }
     }
-    template <class C> __device__ __forceinline__ C load(int b, int p) const {
-        const int o = at<C>(b, p);
-        return o >= 0 ? base[o] : czero<C>();
-    }
-};
+    if constexpr (TT::NPX > 1) __syncthreads();
+}
 
 template <class T, int L, bool TAB, class TT = MvTiles<T, L>, class Pre = PreNone<T>>
 __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_fwd_x(const MvArgs<T> a, const Pre pre, const MvRed red) {
     using C = cplx<T>;
-    constexpr int TL = TT::TLX, NB = TT::NBX, NT = TT::NTX;
+    constexpr int TL = TT::TLX, NB = TT::NBX, NT = TT::NTX, NP = TT::NPX;
     const int rhs = blockIdx.z;
     C* tw = smem_base<C>();
     C* sm = tw + L;
@@ -262,12 +401,15 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_fwd_x(const MvArgs<T> a,
     load_twiddles<C, L, NT>(tw, a.twx);
     pdl_trigger();
     pdl_wait();
-    if (a.status && a.status[rhs]) return;
-    FwdXLoad<T, TAB, Pre> src{a.tab_of(rhs), a.alpha_of(rhs), a.amode, (int)a.nmax, nx, pre, k * nx * ny + j0 * nx,
-                              nl, TL};
+    if (a.status && __ldcg(a.status + rhs)) return;
+    using Src = FwdXLoad<T, TAB, Pre>;
+    Src src{a.tab_of(rhs), a.alpha_of(rhs), a.amode, (int)a.nmax, nx, pre, k * nx * ny + j0 * nx, nl, TL};
     src.pre.bind(a, rhs);
-    B1RowIO<T, L, TL> dst{a.B1 + rhs * a.g.b1_rhs + ((long)k * ny + j0) * L, nl, nz * ny * L};
-    fft_tile<C, L, NB, NT, +1, typename TT::LayX>(sm, tw, src, dst);
+    C* base = a.B1 + rhs * a.g.b1_rhs + ((long)k * ny + j0) * L;
+    if constexpr (NP > 1)
+        stockham_range<C, L, NB, NT, +1, typename TT::LayX, false, NP - 1, 0, 1, Src, SmemIO, PLAN_X>(sm, tw, src,
+                                                                                                       SmemIO{});
+    x_store_pairs<C, L, TT>(sm, tw, src, base, nl, nz * ny * L);
     if constexpr (Pre::ND > 0)
         block_partial<NT, Pre::ND>(src.pre.acc,
                                    red.ppart + (((long)rhs * gridDim.y + k) * red.gxs + blockIdx.x) * Pre::ND);
@@ -275,124 +417,133 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_fwd_x(const MvArgs<T> a,
 
 // ---- pass 2 and 4 ---------------------------------------------------------
 // DIR=+1: B1 (ny rows) -> B2 (Y rows);  DIR=-1: B2 (Y rows) -> B1 (ny rows)
-template <class T, int DIR, int PF = 0> struct YLoad {
+template <class E, int DIR, int PF = 0> struct YLoad {
     static constexpr bool GLOBAL = true, HALF = DIR > 0;  // forward: rows >= ny are padding
-    const cplx<T>* src;
-    int X, i0;
+    const E* src;   // first column of the tile
+    int pitch, nv;  // elements between rows, valid columns
     template <class C> __device__ __forceinline__ C load(int b, int p) const {
-        const int i = i0 + b;
-        return i < X ? ld_l2pf<PF>(src + p * X + i) : czero<C>();
+        return b < nv ? ld_l2pf<PF>(src + p * pitch + b) : czero<C>();
     }
 };
-template <class T, int DIR> struct YStore {
+template <class E, int DIR> struct YStore {
     static constexpr bool GLOBAL = true, HALF = DIR < 0;  // inverse: keep rows < ny
-    cplx<T>* dst;
-    int X, i0;
+    E* dst;
+    int pitch, nv;
     template <class C> __device__ __forceinline__ void store(int b, int p, C v) const {
-        const int i = i0 + b;
-        if (i < X) dst[p * X + i] = v;
+        if (b < nv) dst[p * pitch + b] = v;
     }
 };
 
 template <class T, int L, int DIR, class TT = MvTiles<T, L>>
 __global__ void __launch_bounds__(TT::NTY, TT::MINBY) k_pass_y(const MvArgs<T> a) {
-    using C = cplx<T>;
-    constexpr int TL = TT::TLY, NT = TT::NTY;
-    const int rhs = blockIdx.z / 3, c = blockIdx.z - 3 * (blockIdx.z / 3);
-    C* tw = smem_base<C>();
-    C* sm = tw + L;
-    const int X = a.g.X, ny = a.g.ny, nz = a.g.nz;
+    using E = typename TT::E;
+    using W = cplx<T>;
+    constexpr int TL = TT::TLY, NT = TT::NTY, V = TT::SE / TT::S;  // complex values per element
+    const int rhs = blockIdx.z / 3, c = blockIdx.z - 3 * rhs;
+    W* tw = smem_base<W>();
+    E* sm = reinterpret_cast<E*>(tw + L);
+    const int XE = a.g.X / V, ny = a.g.ny, nz = a.g.nz;
     const int i0 = blockIdx.x * TL, k = blockIdx.y;
-    load_twiddles<C, L, NT>(tw, a.twy);
+    load_twiddles<W, L, NT>(tw, a.twy);
     pdl_trigger();
     pdl_wait();
-    if (a.status && a.status[rhs]) return;
-    const int rows_in = DIR > 0 ? ny : L;
-    const int rows_out = DIR > 0 ? L : ny;
-    const C* srcb = DIR > 0 ? a.B1 + rhs * a.g.b1_rhs : a.B2 + rhs * a.g.b2_rhs;
-    C* dstb = DIR > 0 ? a.B2 + rhs * a.g.b2_rhs : a.B1 + rhs * a.g.b1_rhs;
-    YLoad<T, DIR, TT::ZPF> src{srcb + ((long)c * nz + k) * rows_in * X, X, i0};
-    YStore<T, DIR> dst{dstb + ((long)c * nz + k) * rows_out * X, X, i0};
-    fft_tile<C, L, TL, NT, DIR, typename TT::LayY>(sm, tw, src, dst);
+    if (a.status && __ldcg(a.status + rhs)) return;
+    const int nv = min(TL, XE - i0);
+    E* b1 = reinterpret_cast<E*>(a.B1 + rhs * a.g.b1_rhs) + ((long)c * nz + k) * ny * XE + i0;
+    E* b2 = reinterpret_cast<E*>(a.B2 + rhs * a.g.b2_rhs) + ((long)c * nz + k) * L * XE + i0;
+    YLoad<E, DIR, TT::ZPF> src{DIR > 0 ? b1 : b2, XE, nv};
+    YStore<E, DIR> dst{DIR > 0 ? b2 : b1, XE, nv};
+    fft_tile<E, L, TL, NT, DIR, typename TT::LayY, YLoad<E, DIR, TT::ZPF>, YStore<E, DIR>, PLAN_Y>(sm, tw, src, dst);
 }
 
 // ---- pass 3 -----------------------------------------------------------------
-// lines b = (h * 3 + c) * TL + il: h = 0 row qy, h = 1 the mirror row Y - qy
-template <class T, int TL, int PF = 0> struct ZLoad {
+// lines b = c * TL + il: component c of column il
+template <class E, int TL, int PF = 0> struct ZLoad {
     static constexpr bool GLOBAL = true, HALF = true;  // rows >= nz are padding
-    const cplx<T>* base;  // B2 of this right-hand side, column i0 of row qy
-    int rs;    // elements between z rows (Y * X)
-    int comp;  // elements between components (nz * Y * X)
-    int drow;  // row Y - qy minus row qy
-    int nv, two;  // valid columns, rows in the block (1 or 2)
+    const E* base;  // first column of the tile
+    int rs, comp;   // elements between z rows and between components
+    int nv;         // valid columns
     template <class C> __device__ __forceinline__ C load(int b, int p) const {
-        const int hc = b / TL, il = b - hc * TL;
-        const int h = hc / 3, c = hc - 3 * h;
-        if (il >= nv || h >= two) return czero<C>();
-        return ld_l2pf<PF>(base + c * comp + p * rs + h * drow + il);
+        const int c = b / TL, il = b - c * TL;
+        return il < nv ? ld_l2pf<PF>(base + c * comp + p * rs + il) : czero<C>();
     }
 };
-template <class T, int TL> struct ZStore {
+template <class E, int TL> struct ZStore {
     static constexpr bool GLOBAL = true, HALF = true;  // keep z rows < nz
-    cplx<T>* base;
-    int rs, comp, drow, nv, two;
+    E* base;
+    int rs, comp, nv;
     template <class C> __device__ __forceinline__ void store(int b, int p, C v) const {
-        const int hc = b / TL, il = b - hc * TL;
-        const int h = hc / 3, c = hc - 3 * h;
-        if (il < nv && h < two) base[c * comp + p * rs + h * drow + il] = v;
+        const int c = b / TL, il = b - c * TL;
+        if (il < nv) base[c * comp + p * rs + il] = v;
     }
 };
 
-// Group g of the fused zconv middle -> (column il, butterfly j, mirror row h):
-// order 0 takes il fastest, then j, then h; order 1 il, then h, then j.
-__host__ __device__ constexpr void zmid_map(int order, int g, int TL, int NJ, int& il, int& j, int& h) {
-    il = g % TL;
-    if (order == 0) {
-        j = (g / TL) % NJ;
-        h = g / (TL * NJ);
-    } else {
-        h = (g / TL) % 2;
-        j = g / (2 * TL);
-    }
+// acc + g v with g = s (g.x + i g.y), s = +-1 folded into the products' signs
+__device__ __forceinline__ double2 gfma(double2 acc, double2 g, double s, double2 v) {
+    const double gx = s * g.x, gy = s * g.y;
+    return make_double2(fma(gx, v.x, fma(-gy, v.y, acc.x)), fma(gx, v.y, fma(gy, v.x, acc.y)));
+}
+__device__ __forceinline__ cpair gfma(cpair acc, float2 g, float s, cpair v) {
+    const float gx = s * g.x, gy = s * g.y;
+    const float2 gx2 = make_float2(gx, gx), gy2 = make_float2(gy, gy), ng2 = make_float2(-gy, -gy);
+    return cpair{fma2(gx2, v.re, fma2(ng2, v.im, acc.re)), fma2(gx2, v.im, fma2(gy2, v.re, acc.im))};
+}
+__device__ __forceinline__ double2 gmul(double2 g, double2 v) {
+    return make_double2(fma(g.x, v.x, -g.y * v.y), fma(g.x, v.y, g.y * v.x));
+}
+__device__ __forceinline__ cpair gmul(float2 g, cpair v) {
+    const float2 gx2 = make_float2(g.x, g.x), gy2 = make_float2(g.y, g.y), ng2 = make_float2(-g.y, -g.y);
+    return cpair{fma2(gx2, v.re, mul2(ng2, v.im)), fma2(gx2, v.im, mul2(gy2, v.re))};
+}
+// acc + s g v with one g per value of the pair (the column t = 0: qx = 0, nx)
+__device__ __forceinline__ cpair gfma2(cpair acc, float2 g0, float2 g1, float s, cpair v) {
+    const float2 gx = make_float2(s * g0.x, s * g1.x), gy = make_float2(s * g0.y, s * g1.y);
+    return cpair{fma2(gx, v.re, fma2(make_float2(-gy.x, -gy.y), v.im, acc.re)),
+                 fma2(gx, v.im, fma2(gy, v.re, acc.im))};
 }
 
-// Shared-memory cost of the middle's reads (points j + r NJ) and writes
-// (points j RK + r) under a group order, for the first warps of a block: each
-// request of 32 lanes is served in phases of 128 bytes (16 lanes of 8-byte or
-// 8 lanes of 16-byte elements), and a phase costs the largest number of
-// distinct addresses that share a bank group.  Used at compile time to pick
-// the order without bank conflicts.
-template <class LZ> constexpr int zmid_cost(int order, int TL, int NJ, int RK, int NG, int S) {
-    const int per = 128 / S;
-    int total = 0;
-    for (int w = 0; w < 4 && w * 32 < NG; w++)
-        for (int pass = 0; pass < 2; pass++)
-            for (int r = 0; r < RK; r++)
-                for (int ph = 0; ph < 32 / per; ph++) {
-                    int addr[16] = {};
-                    int n = 0;
-                    for (int l = 0; l < per; l++) {
-                        const int g = w * 32 + ph * per + l;
-                        if (g >= NG) continue;
-                        int il = 0, j = 0, h = 0;
-                        zmid_map(order, g, TL, NJ, il, j, h);
-                        const int p = pass == 0 ? j + r * NJ : j * RK + r;
-                        addr[n++] = LZ::pidx(p) * LZ::PS + h * 3 * TL + il;
-                    }
-                    int worst = 0;
-                    for (int a = 0; a < n; a++) {
-                        int cnt = 0;
-                        for (int q = 0; q < n; q++) {
-                            if (addr[q] % per != addr[a] % per) continue;
-                            bool dup = false;
-                            for (int z = 0; z < q; z++) dup = dup || addr[z] == addr[q];
-                            if (!dup) cnt++;
-                        }
-                        worst = cnt > worst ? cnt : worst;
-                    }
-                    total += worst;
-                }
-    return total;
+// v <- G v for the RK points j + r NJ of one column; g: its slice [c6][qz].
+// Spectral mirrors: z beyond nz flips xz and yz, MY (row Y - qy) xy and yz
+// (component x of a mirrored column is stored negated, so xy and xz need no
+// flip for X - qx).
+template <class E, int L, int RK, bool MY, class W>
+__device__ __forceinline__ void zmultiply(E (&v)[3][RK], const W* g, int j) {
+    using T = typename elem_traits<E>::T;
+    constexpr int NJ = L / RK, NQ = L / 2 + 1;
+    const T sy = MY ? T(-1) : T(1);
+#pragma unroll
+    for (int r = 0; r < RK; r++) {
+        const int p = j + r * NJ;
+        // at 2 p = L the odd components vanish, either sign will do
+        const bool mir = RK % 2 == 0 ? 2 * r >= RK : 2 * p > L;
+        const W* gq = g + (mir ? L - p : p);
+        const T sz = mir ? T(-1) : T(1);
+        const E x = v[0][r], y = v[1][r], z = v[2][r];
+        const W gxy = gq[NQ], gxz = gq[2 * NQ], gyz = gq[4 * NQ];
+        v[0][r] = gfma(gfma(gmul(gq[0], x), gxy, sy, y), gxz, sz, z);
+        v[1][r] = gfma(gfma(gmul(gq[3 * NQ], y), gxy, sy, x), gyz, sy * sz, z);
+        v[2][r] = gfma(gfma(gmul(gq[5 * NQ], z), gxz, sz, x), gyz, sy * sz, y);
+    }
+}
+// the FP32 pair t = 0, whose two values have columns of their own
+template <int L, int RK>
+__device__ __forceinline__ void zmultiply_ends(cpair (&v)[3][RK], const float2* g0, const float2* g1, float sy, int j) {
+    constexpr int NJ = L / RK, NQ = L / 2 + 1;
+#pragma unroll
+    for (int r = 0; r < RK; r++) {
+        const int p = j + r * NJ;
+        const bool mir = 2 * p > L;
+        const int q = mir ? L - p : p;
+        const float sz = mir ? -1.f : 1.f;
+        const cpair x = v[0][r], y = v[1][r], z = v[2][r];
+        const cpair o = czero<cpair>();
+        v[0][r] = gfma2(gfma2(gfma2(o, g0[q], g1[q], 1.f, x), g0[q + NQ], g1[q + NQ], sy, y), g0[q + 2 * NQ],
+                        g1[q + 2 * NQ], sz, z);
+        v[1][r] = gfma2(gfma2(gfma2(o, g0[q + 3 * NQ], g1[q + 3 * NQ], 1.f, y), g0[q + NQ], g1[q + NQ], sy, x),
+                        g0[q + 4 * NQ], g1[q + 4 * NQ], sy * sz, z);
+        v[2][r] = gfma2(gfma2(gfma2(o, g0[q + 5 * NQ], g1[q + 5 * NQ], 1.f, z), g0[q + 2 * NQ], g1[q + 2 * NQ], sz, x),
+                        g0[q + 4 * NQ], g1[q + 4 * NQ], sy * sz, y);
+    }
 }
 
 // Forward z transform (passes 0 .. n-2 of the plan), then in registers: the
@@ -400,92 +551,91 @@ template <class LZ> constexpr int zmid_cost(int order, int TL, int NJ, int RK, i
 // transform run on the reversed plan, so the inverse starts from the values
 // the forward one ended with (its pass 0 reads exactly the points
 // j + r L/R the forward last pass produced), then inverse passes 1 .. n-1.
-// Grid (right-hand side, column tile, mirror-row pair): the right-hand side
-// varies fastest, so the blocks that read one slice of the spectrum run
-// together and a batch takes that slice from HBM once (L2 serves the rest).
-// (A loop over right-hand sides inside the block, keeping the slice in shared
-// memory, needs about twice the registers and spills.)
+//
+// Bound by latency at 12 warps per SM: at 64^3 the FP64 pipe, shared memory and
+// instruction issue are each 35-40% busy.  Against one complex value per
+// thread and element, a slice of the spectrum per column and 2.06e7 warp
+// instructions: FP64 58.1 -> 43.5 us (1.60e7), FP32 35.2 -> 27.9 us (1.95e7 ->
+// 1.06e7: packed sums, one spectrum value for two columns, no work on the
+// padding's zeros).
+// Grid (2 right-hand side + mirror row, column tile, qy): the blocks that read
+// one slice of the spectrum run together, so a batch takes that slice from
+// HBM once (L2 serves the rest).
 template <class T, int L, class TT = MvTiles<T, L>>
 __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a) {
-    using C = cplx<T>;
+    using E = typename TT::E;
+    using W = cplx<T>;
     using LZ = typename TT::LayZ;
-    constexpr int TL = TT::TLZ, NB = TT::NBZ, NT = TT::NTZ;
-    constexpr int ZP = TT::ZP;
-    constexpr int NP = plan_len(L, ZP);
-    constexpr int RK = plan_radix(L, NP - 1, ZP);  // last forward radix = first inverse radix
-    constexpr int NJ = L / RK;                 // butterflies per line in that pass
-    constexpr int MR = TT::MRZ;                // mirror rows per block
-    constexpr int NG = MR * TL * NJ;           // (row half, column, butterfly) groups
+    constexpr int TL = TT::TLZ, NB = TT::NBZ, NT = TT::NTZ, TC = TT::TCZ, GST = TT::GST;
+    constexpr int NP = TT::NPZ;
+    constexpr int RK = TT::RK;                 // last forward radix = first inverse radix
+    constexpr int NJ = TT::NJZ;                // butterflies per line in that pass
+    constexpr int NG = TL * NJ;                // (column, butterfly) groups
     constexpr int PERM = (NG + NT - 1) / NT;
-    constexpr int S = (int)sizeof(C);
-    constexpr int ORDER =
-        MR == 2 && zmid_cost<LZ>(1, TL, NJ, RK, NG, S) < zmid_cost<LZ>(0, TL, NJ, RK, NG, S) ? 1 : 0;
-    constexpr int NQ = L / 2 + 1;
-    // with one mirror row per block, blockIdx.x = 2 rhs + hm: hm = 1 takes
-    // row Y - qy (which exists for 0 < qy < ny only)
-    const int rhs = MR == 2 ? (int)blockIdx.x : (int)blockIdx.x >> 1;
-    const int hm = MR == 2 ? 0 : (int)blockIdx.x & 1;
-    C* tw = smem_base<C>();
-    C* sm = tw + L;
-    C* gs = sm + LZ::span(L) * TT::PSZ;
-    const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz, X = a.g.X, Y = a.g.Y;
+    constexpr int V = TT::SE / TT::S;          // complex values per element
+    // hm = 1 takes row Y - qy (which exists for 0 < qy < ny only)
+    const int rhs = (int)blockIdx.x >> 1, hm = (int)blockIdx.x & 1;
+    W* tw = smem_base<W>();
+    E* sm = reinterpret_cast<E*>(tw + L);
+    W* gs = reinterpret_cast<W*>(sm + LZ::span(L) * NB);
+    const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz, Y = a.g.Y, XE = a.g.X / V;
     const int i0 = blockIdx.y * TL;
     const int qy = blockIdx.z;                    // 0 .. ny
-    const bool pair = qy > 0 && qy < ny;
-    if (hm && !pair) return;
-    const int two = MR == 2 && pair ? 2 : 1;      // rows qy and Y - qy in the block
-    const int row = hm ? Y - qy : qy;             // the block's first row
-    load_twiddles<C, L, NT>(tw, a.twz);
-    const C* gbase = (a.gc_r ? a.gc_r[rhs] : a.Gc) + qy * (nx + 1);
-    // this block's slice of the compressed spectrum (qy fixed, every qz, the
-    // TL columns qx(i)) is copied into shared memory while the forward
-    // transform runs
-    {
-        static_assert(NT % TL == 0, "a thread keeps one column of the slice");
-        const int il = threadIdx.x % TL;
-        const int i = min(i0 + il, X - 1);
-        const int qxc = i <= nx ? i : X - i;
-        const C* gsrc = gbase + qxc;
-        const int gcs = (int)a.g.gc_comp, qzs = (ny + 1) * (nx + 1);
-        for (int cq = threadIdx.x / TL; cq < 6 * NQ; cq += NT / TL) {
-            const int c6 = cq / NQ, qz = cq - c6 * NQ;
-            cp_async_elem<TT::ZPF>(gs + cq * TL + il, gsrc + c6 * gcs + qz * qzs);
+    if (hm && !(qy > 0 && qy < ny)) return;
+    const int t0 = i0 * V / 2;           // first pair of the tile
+    load_twiddles<W, L, NT>(tw, a.twz);
+    // the tile's columns of the compressed spectrum (contiguous each) are
+    // copied into shared memory while the forward transform runs; the last
+    // one is qx = nx, the partner of t = 0
+    const W* gbase = (a.gc_r ? a.gc_r[rhs] : a.Gc) + (long)qy * (nx + 1) * (6 * TT::NQ);
+    if constexpr (!TT::ZSMALL) {
+        constexpr int CH = 6 * TT::NQ * (int)sizeof(W) / 16;
+        static_assert(6 * TT::NQ * sizeof(W) % 16 == 0 && GST * sizeof(W) % 16 == 0, "16-byte copies");
+#pragma unroll
+        for (int col = 0; col <= TC; col++) {
+            const int qx = col < TC ? t0 + col : nx;
+            if (!(col < TC ? qx < nx : t0 == 0)) continue;
+            const char* src = reinterpret_cast<const char*>(gbase + (long)qx * (6 * TT::NQ)) + 16 * threadIdx.x;
+            char* dst = reinterpret_cast<char*>(gs + col * GST) + 16 * threadIdx.x;
+#pragma unroll
+            for (int ch = 0; ch < CH; ch += NT)
+                if (ch + NT <= CH || ch + (int)threadIdx.x < CH) cp_async16(dst + 16 * ch, src + 16 * ch);
         }
+        cp_async_commit();
     }
-    cp_async_commit();
     // the spectrum and the twiddles are constant: only B2 waits for the y pass
     pdl_trigger();
     pdl_wait();
-    if (a.status && a.status[rhs]) {
-        cp_async_wait_all();
+    if (a.status && __ldcg(a.status + rhs)) {
+        if constexpr (!TT::ZSMALL) cp_async_wait_all();
         return;
     }
-    C* B2 = a.B2 + rhs * a.g.b2_rhs + (long)row * X + i0;
-    const int rs = Y * X, comp = nz * Y * X, drow = (Y - 2 * qy) * X, nv = min(TL, X - i0);
-    const ZLoad<T, TL, TT::ZPF> zload{B2, rs, comp, drow, nv, two};
-    const ZStore<T, TL> zstore{B2, rs, comp, drow, nv, two};
+    const int rs = Y * XE, comp = nz * rs, nv = min(TL, XE - i0);
+    E* B2 = reinterpret_cast<E*>(a.B2 + rhs * a.g.b2_rhs) + (long)(hm ? Y - qy : qy) * XE + i0;
+    const ZLoad<E, TL, TT::ZPF> zload{B2, rs, comp, nv};
+    const ZStore<E, TL> zstore{B2, rs, comp, nv};
     if constexpr (NP > 1)
-        stockham_range<C, L, NB, NT, +1, LZ, false, NP - 1, 0, 1, ZLoad<T, TL, TT::ZPF>, SmemIO, ZP>(sm, tw, zload,
-                                                                                                    SmemIO{});
-    cp_async_wait_all();
-    __syncthreads();
+        stockham_range<E, L, NB, NT, +1, LZ, false, NP - 1, 0, 1, ZLoad<E, TL, TT::ZPF>, SmemIO, TT::PZ>(
+            sm, tw, zload, SmemIO{});
+    if constexpr (!TT::ZSMALL) {
+        cp_async_wait_all();
+        __syncthreads();
+    }
     // ---- fused middle: read, transform, multiply, transform (registers) ----
-    C v[PERM][3][RK];
+    E v[PERM][3][RK];
 #pragma unroll
     for (int q = 0; q < PERM; q++) {
         const int g = threadIdx.x + q * NT;
         if (!(PERM * NT == NG || g < NG)) continue;
-        int il, j, h;
-        zmid_map(ORDER, g, TL, NJ, il, j, h);
-        const int i = i0 + il;
+        const int il = g % TL, j = g / TL;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            const int b = (h * 3 + c) * TL + il;
+            const int b = c * TL + il;
 #pragma unroll
             for (int r = 0; r < RK; r++) {
                 const int p = j + r * NJ;
                 if constexpr (NP == 1) {
-                    v[q][c][r] = (2 * p >= L) ? czero<C>() : zload.template load<C>(b, p);
+                    v[q][c][r] = (2 * p >= L) ? czero<E>() : zload.template load<E>(b, p);
                 } else if constexpr (read_split<LZ>(NJ, RK)) {
                     v[q][c][r] = sm[LZ::addr(j, b) + LZ::pidx(r * NJ) * LZ::PS];
                 } else {
@@ -497,51 +647,42 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
 #pragma unroll
                 for (int r = 1; r < RK; r++) v[q][c][r] = cmul(v[q][c][r], tw[j * r]);
             }
-            Dft<RK, +1, C>::run(v[q][c]);
+            Dft<RK, +1, E>::run(v[q][c]);
         }
-        if (h < two && i < X) {
-            const T sx = i <= nx ? (T)1 : (T)-1;
-            const T sy = (h | hm) ? (T)-1 : (T)1;
-#pragma unroll
-            for (int r = 0; r < RK; r++) {
-                const int p = j + r * NJ;  // spectral index of this output
-                const int qzc = 2 * p <= L ? p : L - p;  // nz = L / 2
-                const T sz = 2 * p <= L ? (T)1 : (T)-1;
-                C g6[6];
-                const C* gq = gs + qzc * TL + il;
-#pragma unroll
-                for (int c6 = 0; c6 < 6; c6++) g6[c6] = gq[c6 * NQ * TL];
-                const C gxx = g6[0];
-                const C gxy = cscale(g6[1], sx * sy);
-                const C gxz = cscale(g6[2], sx * sz);
-                const C gyy = g6[3];
-                const C gyz = cscale(g6[4], sy * sz);
-                const C gzz = g6[5];
-                const C vx = v[q][0][r], vy = v[q][1][r], vz = v[q][2][r];
-                v[q][0][r] = cadd(cadd(cmul(gxx, vx), cmul(gxy, vy)), cmul(gxz, vz));
-                v[q][1][r] = cadd(cadd(cmul(gxy, vx), cmul(gyy, vy)), cmul(gyz, vz));
-                v[q][2][r] = cadd(cadd(cmul(gxz, vx), cmul(gyz, vy)), cmul(gzz, vz));
+        if (il < nv) {
+            const int t = V == 2 ? il : il >> 1;  // column of the slice
+            const bool ends = V == 2 ? t0 + t == 0 : (t0 == 0 && il == 1);
+            if constexpr (V == 2) {
+                const W* g0 = TT::ZSMALL ? gbase + (long)(t0 + t) * (6 * TT::NQ) : gs + t * GST;
+                if (ends)
+                    zmultiply_ends<L, RK>(v[q], g0, TT::ZSMALL ? gbase + (long)nx * (6 * TT::NQ) : gs + TC * GST,
+                                          hm ? -1.f : 1.f, j);
+                else if (hm) zmultiply<E, L, RK, true>(v[q], g0, j);
+                else zmultiply<E, L, RK, false>(v[q], g0, j);
+            } else {
+                const W* gcol = TT::ZSMALL ? gbase + (long)(ends ? nx : t0 + t) * (6 * TT::NQ) : gs + (ends ? TC : t) * GST;
+                if (hm) zmultiply<E, L, RK, true>(v[q], gcol, j);
+                else zmultiply<E, L, RK, false>(v[q], gcol, j);
             }
         }
         // inverse pass 0 of the reversed plan: Ns = 1, inputs j + r NJ, no twiddles
 #pragma unroll
-        for (int c = 0; c < 3; c++) Dft<RK, -1, C>::run(v[q][c]);
+        for (int c = 0; c < 3; c++) Dft<RK, -1, E>::run(v[q][c]);
     }
     if constexpr (NP > 1) __syncthreads();  // every read of the tile is done
 #pragma unroll
     for (int q = 0; q < PERM; q++) {
         const int g = threadIdx.x + q * NT;
         if (!(PERM * NT == NG || g < NG)) continue;
-        int il, j, h;
-        zmid_map(ORDER, g, TL, NJ, il, j, h);
+        const int il = g % TL, j = g / TL;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            const int b = (h * 3 + c) * TL + il;
+            const int b = c * TL + il;
 #pragma unroll
             for (int r = 0; r < RK; r++) {
                 const int o = j * RK + r;
                 if constexpr (NP == 1) {
-                    if (2 * o < L) zstore.template store<C>(b, o, v[q][c][r]);
+                    if (2 * o < L) zstore.template store<E>(b, o, v[q][c][r]);
                 } else if constexpr (write_split<LZ>(NJ, 1, RK)) {
                     sm[LZ::addr(j * RK, b) + LZ::pidx(r) * LZ::PS] = v[q][c][r];
                 } else {
@@ -552,7 +693,8 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
     }
     if constexpr (NP > 1) {
         __syncthreads();
-        stockham_range<C, L, NB, NT, -1, LZ, true, NP, 1, RK, SmemIO, ZStore<T, TL>, ZP>(sm, tw, SmemIO{}, zstore);
+        stockham_range<E, L, NB, NT, -1, LZ, true, NP, 1, RK, SmemIO, ZStore<E, TL>, TT::PZ>(sm, tw, SmemIO{},
+                                                                                            zstore);
     }
 }
 
@@ -607,12 +749,15 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_inv_x(const MvArgs<T> a,
     load_twiddles<C, L, NT>(tw, a.twx);
     pdl_trigger();
     pdl_wait();
-    if (a.status && a.status[rhs]) return;
-    B1RowIO<T, L, TL> src{a.B1 + rhs * a.g.b1_rhs + ((long)k * ny + j0) * L, nl, nz * ny * L};
+    if (a.status && __ldcg(a.status + rhs)) return;
+    const C* base = a.B1 + rhs * a.g.b1_rhs + ((long)k * ny + j0) * L;
     InvXStore<T, TAB, Epi> dst{a.tab_of(rhs), a.b + rhs * a.xstride, a.y + rhs * a.xstride, a.inv_m, nx,
                                k * nx * ny + j0 * nx, nl, TL, epi};
     dst.epi.bind(a, rhs);
-    fft_tile<C, L, NB, NT, -1, typename TT::LayX>(sm, tw, src, dst);
+    x_load_pairs<C, L, TT>(sm, dst, base, nl, nz * ny * L);
+    if constexpr (TT::NPX > 1)
+        stockham_range<C, L, NB, NT, -1, typename TT::LayX, true, TT::NPX, 1, TT::RX, SmemIO, InvXStore<T, TAB, Epi>,
+                       PLAN_X>(sm, tw, SmemIO{}, dst);
     if constexpr (Epi::ND > 0) {
         double2 tot[Epi::ND + Epi::NDP];
         if (reduce_rows<NT, Epi::ND, Epi::NDP>(dst.epi.acc, tot, rhs, blockIdx.x, k, gridDim.x, gridDim.y, red) &&
