@@ -100,27 +100,45 @@ __device__ __forceinline__ void ydft_plane(const MicGeom& m, const double2* __re
 //          exp(-i (var1 i + var2 j)) / (-2 pi i kz)
 // with the products and sums of the pupil test and of kz rounded one by one
 // as the reference evaluates them.
-__global__ void __launch_bounds__(256) k_mic_far(const MicGeom m, int nb, const double2* __restrict__ Q,
-                                                  const double* __restrict__ zplane, const double2* __restrict__ tw,
-                                                  double2* __restrict__ Ed) {
+//
+// One pupil point reads nz ny values of Q one after the other, and there are
+// only nb S^2 points (1690 for 10 illuminations of a 24^3 object: 7 blocks of
+// one thread per point took 319 us, latency of a serial chain).  So a block
+// takes FAR_P points and cuts their planes into FAR_G shares, summed in order
+// at the end.
+constexpr int FAR_P = 16, FAR_G = 16;
+// adds the FAR_G shares of each of a block's points in order, into thread g = 0's acc
+template <int N> __device__ __forceinline__ void far_sum(double2 (&acc)[N], int p, int g) {
+    __shared__ double2 part[FAR_G][FAR_P][N];
+#pragma unroll
+    for (int c = 0; c < N; c++) part[g][p][c] = acc[c];
+    __syncthreads();
+    if (g > 0) return;
+    for (int h = 1; h < FAR_G; h++)
+#pragma unroll
+        for (int c = 0; c < N; c++) acc[c] = cadd(acc[c], part[h][p][c]);
+}
+__global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far(const MicGeom m, int nb, const double2* __restrict__ Q,
+                                                            const double* __restrict__ zplane,
+                                                            const double2* __restrict__ tw, double2* __restrict__ Ed) {
     const int S = m.S();
     const long total = (long)nb * S * S;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
+    const int p = threadIdx.x % FAR_P, g = threadIdx.x / FAR_P;
+    const long t = (long)blockIdx.x * FAR_P + p;
     const int irow = (int)(t % S);
     const int jrow = (int)((t / S) % S);
     const int b = (int)(t / ((long)S * S));
     const int i = irow - m.imax, j = jrow - m.imax, n = m.n;
     const double kx = (double)i * m.dkx, ky = (double)j * m.dky;
-    double2 o0 = make_double2(0, 0), o1 = o0, o2 = o0;
-    if (__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)) < __dmul_rn(m.numaper, m.numaper)) {
+    double2 o[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+    if (t < total && __dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)) < __dmul_rn(m.numaper, m.numaper)) {
         const double kz = sqrt(__dsub_rn(__dsub_rn(__dmul_rn(m.k0, m.k0), __dmul_rn(kx, kx)), __dmul_rn(ky, ky)));
         double sn, cs;
         sincos(-__dadd_rn(__dmul_rn(m.var1, (double)i), __dmul_rn(m.var2, (double)j)), &sn, &cs);
         const double2 exy = make_double2(cs, sn);
         const double2 den = make_double2(0.0, -2.0 * 3.14159265358979323846 * kz);
         const int step = posmod(j, n), ph0 = posmod((long)j * (-(n / 2)), n);
-        for (int k = 0; k < m.nz; k++) {
+        for (int k = g * m.nz / FAR_G; k < (g + 1) * m.nz / FAR_G; k++) {
             double2 p0, p1, p2;
             ydft_plane(m, Q, tw, b, k, irow, ph0, step, p0, p1, p2);
             // ctmp = (kx P_x + ky P_y + kz dside P_z) / k0, on the side dside
@@ -129,19 +147,19 @@ __global__ void __launch_bounds__(256) k_mic_far(const MicGeom m, int nb, const 
                                             (kx * p0.y + ky * p1.y + kzs * p2.y) / m.k0);
             sincos(-kzs * zplane[k], &sn, &cs);
             const double2 c1 = zdiv(cmul(make_double2(cs, sn), exy), den);
-            o0 = cadd(o0, cmul(csub(p0, make_double2(kx * ct.x / m.k0, kx * ct.y / m.k0)), c1));
-            o1 = cadd(o1, cmul(csub(p1, make_double2(ky * ct.x / m.k0, ky * ct.y / m.k0)), c1));
-            o2 = cadd(o2, cmul(csub(p2, make_double2(kzs * ct.x / m.k0, kzs * ct.y / m.k0)), c1));
+            o[0] = cadd(o[0], cmul(csub(p0, make_double2(kx * ct.x / m.k0, kx * ct.y / m.k0)), c1));
+            o[1] = cadd(o[1], cmul(csub(p1, make_double2(ky * ct.x / m.k0, ky * ct.y / m.k0)), c1));
+            o[2] = cadd(o[2], cmul(csub(p2, make_double2(kzs * ct.x / m.k0, kzs * ct.y / m.k0)), c1));
         }
         const double k02 = m.k0 * m.k0;
-        o0 = cscale(o0, k02);
-        o1 = cscale(o1, k02);
-        o2 = cscale(o2, k02);
+#pragma unroll
+        for (int c = 0; c < 3; c++) o[c] = cscale(o[c], k02);
     }
-    double2* e = Ed + (((long)b * S + jrow) * S + irow) * 3;
-    e[0] = o0;
-    e[1] = o1;
-    e[2] = o2;
+    far_sum<3>(o, p, g);
+    if (g > 0 || t >= total) return;
+    double2* e = Ed + t * 3;
+#pragma unroll
+    for (int c = 0; c < 3; c++) e[c] = o[c];
 }
 
 // Far field on both sides without a lens (diffractefft2d.f:104-170): for
@@ -149,27 +167,29 @@ __global__ void __launch_bounds__(256) k_mic_far(const MicGeom m, int nb, const 
 //   E+_c = sum_k (P_c - k+_c (k+.P) / k0^2) exp(-i kz z_k) exp(-i (var1 i + var2 j))
 //   E-_c = sum_k (P_c - k-_c (k-.P) / k0^2) exp(+i kz z_k) exp(-i (var1 i + var2 j))
 // with k+- = (kx, ky, +-kz); Ed holds E+ for all nb, then E-.
-__global__ void __launch_bounds__(256) k_mic_far2(const MicGeom m, int nb, const double2* __restrict__ Q,
-                                                   const double* __restrict__ zplane, const double2* __restrict__ tw,
-                                                   double2* __restrict__ Ed) {
+__global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far2(const MicGeom m, int nb, const double2* __restrict__ Q,
+                                                             const double* __restrict__ zplane,
+                                                             const double2* __restrict__ tw, double2* __restrict__ Ed) {
     const int S = m.S();
     const long total = (long)nb * S * S;
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
+    const int p = threadIdx.x % FAR_P, g = threadIdx.x / FAR_P;
+    const long t = (long)blockIdx.x * FAR_P + p;
     const int irow = (int)(t % S);
     const int jrow = (int)((t / S) % S);
     const int b = (int)(t / ((long)S * S));
     const int i = irow - m.imax, j = jrow - m.imax, n = m.n;
     const double kx = (double)i * m.dkx, ky = (double)j * m.dky;
-    double2 a0 = make_double2(0, 0), a1 = a0, a2 = a0, c0 = a0, c1 = a0, c2 = a0;
+    double2 o[6];  // E+, then E-
+#pragma unroll
+    for (int c = 0; c < 6; c++) o[c] = make_double2(0, 0);
     const double kz2 = __dsub_rn(__dsub_rn(__dmul_rn(m.k0, m.k0), __dmul_rn(kx, kx)), __dmul_rn(ky, ky));
-    if (kz2 > 0.0) {
+    if (t < total && kz2 > 0.0) {
         const double kz = sqrt(kz2);
         double sn, cs;
         sincos(-__dadd_rn(__dmul_rn(m.var1, (double)i), __dmul_rn(m.var2, (double)j)), &sn, &cs);
         const double2 exy = make_double2(cs, sn);
         const int step = posmod(j, n), ph0 = posmod((long)j * (-(n / 2)), n);
-        for (int k = 0; k < m.nz; k++) {
+        for (int k = g * m.nz / FAR_G; k < (g + 1) * m.nz / FAR_G; k++) {
             double2 p0, p1, p2;
             ydft_plane(m, Q, tw, b, k, irow, ph0, step, p0, p1, p2);
             sincos(kz * zplane[k], &sn, &cs);
@@ -178,22 +198,23 @@ __global__ void __launch_bounds__(256) k_mic_far2(const MicGeom m, int nb, const
                                             (kx * p0.y + ky * p1.y + kz * p2.y) / m.k0);
             const double2 tn = make_double2((kx * p0.x + ky * p1.x - kz * p2.x) / m.k0,
                                             (kx * p0.y + ky * p1.y - kz * p2.y) / m.k0);
-            a0 = cadd(a0, cmul(csub(p0, make_double2(kx * tp.x / m.k0, kx * tp.y / m.k0)), up));
-            a1 = cadd(a1, cmul(csub(p1, make_double2(ky * tp.x / m.k0, ky * tp.y / m.k0)), up));
-            a2 = cadd(a2, cmul(csub(p2, make_double2(kz * tp.x / m.k0, kz * tp.y / m.k0)), up));
-            c0 = cadd(c0, cmul(csub(p0, make_double2(kx * tn.x / m.k0, kx * tn.y / m.k0)), dn));
-            c1 = cadd(c1, cmul(csub(p1, make_double2(ky * tn.x / m.k0, ky * tn.y / m.k0)), dn));
-            c2 = cadd(c2, cmul(cadd(p2, make_double2(kz * tn.x / m.k0, kz * tn.y / m.k0)), dn));
+            o[0] = cadd(o[0], cmul(csub(p0, make_double2(kx * tp.x / m.k0, kx * tp.y / m.k0)), up));
+            o[1] = cadd(o[1], cmul(csub(p1, make_double2(ky * tp.x / m.k0, ky * tp.y / m.k0)), up));
+            o[2] = cadd(o[2], cmul(csub(p2, make_double2(kz * tp.x / m.k0, kz * tp.y / m.k0)), up));
+            o[3] = cadd(o[3], cmul(csub(p0, make_double2(kx * tn.x / m.k0, kx * tn.y / m.k0)), dn));
+            o[4] = cadd(o[4], cmul(csub(p1, make_double2(ky * tn.x / m.k0, ky * tn.y / m.k0)), dn));
+            o[5] = cadd(o[5], cmul(cadd(p2, make_double2(kz * tn.x / m.k0, kz * tn.y / m.k0)), dn));
         }
     }
-    double2* e = Ed + (((long)b * S + jrow) * S + irow) * 3;
-    e[0] = a0;
-    e[1] = a1;
-    e[2] = a2;
+    far_sum<6>(o, p, g);
+    if (g > 0 || t >= total) return;
+    double2* e = Ed + t * 3;
     double2* f = e + (long)nb * S * S * 3;
-    f[0] = c0;
-    f[1] = c1;
-    f[2] = c2;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        e[c] = o[c];
+        f[c] = o[3 + c];
+    }
 }
 
 // The lens's far field by direct summation over the dipoles (nquicklens = 0,
@@ -589,8 +610,8 @@ void mic_farfield_dev(const MicGeom& m, int nb, const double2* FF, const double*
     k_mic_xdft<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(m, nb, FF, tw, Q);
     IFDDA_CUDA(cudaGetLastError());
     count_launch();
-    if (both_sides) k_mic_far2<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(m, nb, Q, zplane, tw, Ed);
-    else k_mic_far<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(m, nb, Q, zplane, tw, Ed);
+    if (both_sides) k_mic_far2<<<(unsigned)((ne + FAR_P - 1) / FAR_P), FAR_P * FAR_G, 0, st>>>(m, nb, Q, zplane, tw, Ed);
+    else k_mic_far<<<(unsigned)((ne + FAR_P - 1) / FAR_P), FAR_P * FAR_G, 0, st>>>(m, nb, Q, zplane, tw, Ed);
     IFDDA_CUDA(cudaGetLastError());
 }
 
