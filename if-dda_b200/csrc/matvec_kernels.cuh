@@ -102,6 +102,10 @@ template <class T> struct MvArgs {
 //    fit: FP32 at 192^3 1.21 -> 0.89 ms.  Below, where two passes leave 12 warps
 //    or more, three were slower (FP64 at 64^3 57.9 against 45.2 us: the extra
 //    round trip through shared memory).
+// Register caps of the y passes and of zconv's small middles (RK up to 5): 102
+// (five warps per quarter SM; 84 for first radices up to 8) instead of 128:
+// 12 right-hand sides of 48x40x32 in FP64 5.51 -> 5.24 ms a solve, 75x45x29 x2
+// 86.7 -> 84.9 us a mat-vec.
 // The variants are compiled for lengths of 64 and more; the tile chooser
 // (tune_tiles) times both on the caller's grid and keeps one per grid.  The
 // two agree to rounding.
@@ -195,8 +199,8 @@ template <class T, int L, int V = 0> struct MvTiles {
     using LayY = Layout<NBY, 1, true>;
     using LayZ = Layout<NBZ, 1, true, zpadsh(TLZ), zpadoff(TLZ)>;
     static constexpr int MINBX = minblocks(NTX, S == 8 ? 80 : (RX > 8 ? 128 : 102));
-    static constexpr int MINBY = minblocks(NTY, RY == 32 ? 168 : 128);
-    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : 128));
+    static constexpr int MINBY = minblocks(NTY, RY == 32 ? 168 : 102);
+    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : (RZ == 16 ? 102 : 84)));
     static constexpr size_t smem_x = (size_t)L * S + (size_t)NBX * LP * S;
     static constexpr size_t smem_y = (size_t)L * S + (size_t)L * NBY * SE;
     static constexpr size_t smem_z = zbytes(TLZ);
