@@ -37,8 +37,9 @@ __device__ __forceinline__ void block_sum(double2 (&acc)[ND], double2* scratch) 
 #pragma unroll
         for (int m = 0; m < ND; m++) {
             double2 v = lane < NW ? scratch[m * 32 + lane] : make_double2(0, 0);
+            constexpr int O = NW > 16 ? 16 : NW > 8 ? 8 : NW > 4 ? 4 : NW > 2 ? 2 : NW > 1 ? 1 : 0;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = dadd(v, shfl_down2(v, o));
+            for (int o = O; o > 0; o >>= 1) v = dadd(v, shfl_down2(v, o));
             acc[m] = v;
         }
     }
@@ -104,10 +105,15 @@ __device__ __forceinline__ void block_partial(double2 (&acc)[ND], double2* out) 
     }
 }
 
-// Two ticket levels: the last block of a row sums that row's ND partials and
-// the row's NDP partials of the first pass; the last row sums the rows.  All
-// sums run in index order, so the result does not depend on scheduling.
+// Up to FLAT_BLOCKS blocks per right-hand side: one ticket, the last block sums
+// every block's ND partials and the NDP of the first pass.  Above, where that
+// block would read too much, two ticket levels: the last block of a row sums
+// that row, the last row sums the rows.  A level costs the end of the kernel a
+// store, a fence, an atomic and a load one after the other, about 2 us of
+// latency that nothing else hides.  All sums run in index order, so the result
+// does not depend on scheduling; which form is taken depends on the lattice only.
 // Returns true in the one block that holds the totals (thread 0's tot).
+constexpr int FLAT_BLOCKS = 1024;
 template <int NT, int ND, int NDP>
 __device__ __forceinline__ bool reduce_rows(double2 (&own)[ND], double2 (&tot)[ND + NDP], int rhs, int bx, int by,
                                             int gx, int gy, const MvRed& R) {
@@ -116,17 +122,31 @@ __device__ __forceinline__ bool reduce_rows(double2 (&own)[ND], double2 (&tot)[N
     __shared__ bool last;
     block_sum<NT, ND>(own, scratch);
     const long row = (long)rhs * gy + by;
+    const bool flat = gx * gy <= FLAT_BLOCKS;
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int m = 0; m < ND; m++) R.epart[(row * R.gxs + bx) * ND + m] = own[m];
         __threadfence();
-        last = atomicAdd(&R.t1[row], 1u) == (unsigned)(gx - 1);
+        last = flat ? atomicAdd(&R.t2[rhs], 1u) == (unsigned)(gx * gy - 1)
+                    : atomicAdd(&R.t1[row], 1u) == (unsigned)(gx - 1);
     }
     __syncthreads();
     if (!last) return false;
     __threadfence();
 #pragma unroll
     for (int m = 0; m < NA; m++) tot[m] = make_double2(0, 0);
+    if (flat) {
+        for (int i = threadIdx.x; i < gx * gy; i += NT) {
+            const long q = ((long)rhs * gy + i / gx) * R.gxs + i % gx;
+#pragma unroll
+            for (int m = 0; m < ND; m++) tot[m] = dadd(tot[m], __ldcg(R.epart + q * ND + m));
+#pragma unroll
+            for (int m = 0; m < NDP; m++) tot[ND + m] = dadd(tot[ND + m], __ldcg(R.ppart + q * NDP + m));
+        }
+        block_sum<NT, NA>(tot, scratch);
+        if (threadIdx.x == 0) R.t2[rhs] = 0u;
+        return true;
+    }
     for (int q = threadIdx.x; q < gx; q += NT) {
 #pragma unroll
         for (int m = 0; m < ND; m++) tot[m] = dadd(tot[m], __ldcg(R.epart + (row * R.gxs + q) * ND + m));
