@@ -58,7 +58,7 @@ template <class T> struct EpiGpAlpha {
         r0 = V.v(G_R0, rhs);
         acc[0] = make_double2(0, 0);
     }
-    template <int NT> __device__ __forceinline__ void ahead(int e0, int n) const { prefetch_l2<NT>(r0, e0, n); }
+    __device__ __forceinline__ void ahead(int e) const { prefetch_l2(r0 + e); }
     template <class C> __device__ __forceinline__ void elem(int e, C y) {
         acc[0] = zadd(acc[0], zconjmul(ldg(r0, e), to_d(y)));
     }
@@ -119,7 +119,7 @@ template <class T> struct EpiGpZeta {
         acc[0] = acc[1] = acc[2] = make_double2(0, 0);
     }
     // t is the subtrahend b of this mat-vec
-    template <int NT> __device__ __forceinline__ void ahead(int e0, int n) const { prefetch_l2<NT>(y, e0, n); }
+    __device__ __forceinline__ void ahead(int e) const { prefetch_l2(y + e); }
     template <class C> __device__ __forceinline__ void elem(int e, C atc) {
         const double2 a = to_d(atc);
         acc[0] = zadd(acc[0], zconjmul(a, a));

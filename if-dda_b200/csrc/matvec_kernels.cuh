@@ -708,20 +708,20 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
 // the grid then holds them, with the NDP partials of the first x pass, and
 // calls Epi::finish.
 //
-// On a full box the vectors that a tile's last pass reads are known from the
-// start: b and the Epi's own (Epi::ahead) are asked into L2 before the
-// transform, which then runs while they come from DRAM (64^3 FP64 solve 4.92 ->
-// 4.80 ms).
-template <int NT, class C> __device__ __forceinline__ void prefetch_l2(const C* p, int e0, int n) {
-    constexpr int STEP = 128 / (int)sizeof(C);
-    for (int i = threadIdx.x * STEP; i < n; i += NT * STEP)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + e0 + i));
+// The vectors that a tile's last pass reads are known from the start: b and the
+// Epi's own (Epi::ahead) are asked into L2 before the transform, which then
+// runs while they come from DRAM (FP64 solves: 64^3 4.92 -> 4.80 ms, 12
+// right-hand sides of an ellipsoid on 48x40x32 5.35 -> 5.28 ms).  ahead() is
+// called for the first element of a dipole; the three components of one lie
+// within 48 bytes.
+template <class C> __device__ __forceinline__ void prefetch_l2(const C* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 struct EpiNone {
     static constexpr int ND = 0, NDP = 0;
     double2 acc[1];
     template <class T> __device__ __forceinline__ void bind(const MvArgs<T>&, int) {}
-    template <int NT> __device__ __forceinline__ void ahead(int, int) const {}
+    __device__ __forceinline__ void ahead(int) const {}
     template <class C> __device__ __forceinline__ void elem(int, C) {}
     __device__ __forceinline__ void finish(int, const double2*) {}
 };
@@ -769,10 +769,13 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_inv_x(const MvArgs<T> a,
     InvXStore<T, TAB, Epi> dst{a.tab_of(rhs), a.b + rhs * a.xstride, a.y + rhs * a.xstride, a.inv_m, nx,
                                k * nx * ny + j0 * nx, nl, TL, epi};
     dst.epi.bind(a, rhs);
-    if constexpr (!TAB) {
-        const int e0 = 3 * dst.site0, n = 3 * nl * nx;
-        prefetch_l2<NT>(dst.bv, e0, n);
-        dst.epi.template ahead<NT>(e0, n);
+    // one prefetch per dipole with a Tabdip, per 128 bytes without
+    constexpr int STEP = TAB ? 1 : 128 / (3 * (int)sizeof(C));
+    for (int i = threadIdx.x * STEP; i < nl * nx; i += NT * STEP) {
+        const int d = TAB ? __ldg(dst.tab + dst.site0 + i) - 1 : dst.site0 + i;
+        if (d < 0) continue;
+        prefetch_l2(dst.bv + 3 * d);
+        dst.epi.ahead(3 * d);
     }
     x_load_pairs<C, L, TT>(sm, dst, base, nl, nz * ny * L);
     if constexpr (TT::NPX > 1)
