@@ -92,7 +92,9 @@ template <class T> struct MvArgs {
 //    small lattice would otherwise leave SMs without a block).  FP32 keeps to 80
 //    registers: at 96 the 1024 blocks of a 64^3 grid no longer fit the SMs at
 //    once, and the solver's passes took 24.9 instead of 18.5 us;
-//  * y passes: 8 columns of 16 bytes, 16 (V = 1);
+//  * y passes: 16 columns of 16 bytes from length 64 on, 8 below and for V = 1
+//    (FP64 there and back at 64^3 34.5 against 36.6 us; 8 leave a small
+//    lattice more blocks);
 //  * zconv: 8 columns of 16 bytes, rows of 128 bytes.  4 columns (V = 1 below
 //    160) and 2 give more and smaller blocks, but their narrower rows cost more
 //    than that: FP64 at 64^3 43.5, 47.5 and 65 us, FP32 27.9, 29.5 and 40.5 us.
@@ -121,7 +123,7 @@ template <class T, int L, int V = 0> struct MvTiles {
     static constexpr int SE = (int)sizeof(E);
     static constexpr int SMEM_X = L >= 64 ? 16384 : 8192;
     static constexpr int TLX = clamp_pow2(SMEM_X / (3 * (L + 1) * S), 1, 16);
-    static constexpr int TLY = V ? 16 : 8;
+    static constexpr int TLY = V == 0 && L >= 64 ? 16 : 8;
     static constexpr int NBX = 3 * TLX, NBY = TLY;
     // x tile: points contiguous with one pad word every 16, line pitch = 8 (mod 16)
     static constexpr int lpitch() {
