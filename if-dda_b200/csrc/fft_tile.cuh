@@ -494,8 +494,9 @@ template <class Lay> constexpr bool write_split(int NJ, int Ns, int R) {
     return true;
 }
 
-// One Stockham pass.  tw[j] = exp(+2 pi i j / L) in shared memory.
-template <class C, int L, int R, int Ns, int NB, int NT, int DIR, class Lay, class Src, class Dst>
+// One Stockham pass.  tw[j] = exp(+2 pi i j / L) in shared memory.  SYNC: a pass
+// that writes the tile ends in a barrier (otherwise the caller's next one does).
+template <class C, int L, int R, int Ns, int NB, int NT, int DIR, class Lay, class Src, class Dst, bool SYNC = true>
 __device__ __forceinline__ void stockham_pass(C* sm, const typename elem_traits<C>::W* tw, const Src& src,
                                               const Dst& dst, const int tid) {
     using W = typename elem_traits<C>::W;
@@ -575,7 +576,7 @@ __device__ __forceinline__ void stockham_pass(C* sm, const typename elem_traits<
         for (int q = 0; q < PER; q++)
             if (PER * NT == NBF || tid + q * NT < NBF) write(v[q], tid + q * NT);
     }
-    if (!GOUT) __syncthreads();
+    if (!GOUT && SYNC) __syncthreads();
 }
 
 // Passes q in [q, Q1) of the plan (reversed when REV); Ns is the product of

@@ -471,7 +471,7 @@ template <class E, int TL, int PF = 0> struct ZLoad {
     int nv;         // valid columns
     template <class C> __device__ __forceinline__ C load(int b, int p) const {
         const int c = b / TL, il = b - c * TL;
-        return il < nv ? ld_l2pf<PF>(base + c * comp + p * rs + il) : czero<C>();
+        return ld_l2pf<PF>(base + c * comp + p * rs + min(il, nv - 1));  // columns beyond the last are not stored
     }
 };
 template <class E, int TL> struct ZStore {
@@ -620,10 +620,15 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
     E* B2 = reinterpret_cast<E*>(a.B2 + rhs * a.g.b2_rhs) + (long)(hm ? Y - qy : qy) * XE + i0;
     const ZLoad<E, TL, TT::ZPF> zload{B2, rs, comp, nv};
     const ZStore<E, TL> zstore{B2, rs, comp, nv};
-    if constexpr (NP > 1)
-        stockham_range<E, L, NB, NT, +1, LZ, false, NP - 1, 0, 1, ZLoad<E, TL, TT::ZPF>, SmemIO, TT::PZ>(
-            sm, tw, zload, SmemIO{});
-    if constexpr (!TT::ZSMALL) {
+    if constexpr (NP > 1) {
+        stockham_pass<E, L, TT::RZ, 1, NB, NT, +1, LZ, ZLoad<E, TL, TT::ZPF>, SmemIO, false>(sm, tw, zload, SmemIO{},
+                                                                                           threadIdx.x);
+        if constexpr (!TT::ZSMALL && NP == 2) cp_async_wait_all();
+        __syncthreads();
+        stockham_range<E, L, NB, NT, +1, LZ, false, NP - 1, 1, TT::RZ, SmemIO, SmemIO, TT::PZ>(sm, tw, SmemIO{},
+                                                                                              SmemIO{});
+    }
+    if constexpr (!TT::ZSMALL && NP != 2) {
         cp_async_wait_all();
         __syncthreads();
     }
