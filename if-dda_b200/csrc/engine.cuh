@@ -236,7 +236,7 @@ MvArgs<T> mv_args(Green& G, int nrhs, const cplx<T>* x, const cplx<T>* b, cplx<T
 }
 
 // time the tile variants of T on G's grid once (with nrhs right-hand sides),
-// see mv_impl.cuh
+// see yz_impl.cuh
 template <class T> void tune_tiles(Green& G, int nrhs, cudaStream_t st);
 
 }  // namespace ifdda
