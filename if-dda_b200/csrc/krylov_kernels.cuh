@@ -58,7 +58,8 @@ template <class C> __device__ __forceinline__ double2 ld(const C* p, long i) { r
 // The same through the read-only path.  For vectors that a kernel reads at an
 // element before (or without) writing that element from the same thread: the
 // loads may then be issued ahead of the stores to other elements, instead of
-// waiting behind them for want of alias information.
+// waiting behind them for want of alias information.  No other kernel writes
+// them meanwhile: see pdl_trigger().
 template <class C> __device__ __forceinline__ double2 ldg(const C* p, long i) { return to_d(__ldg(p + i)); }
 template <class C> __device__ __forceinline__ void st(C* p, long i, double2 v) { p[i] = from_d<C>(v); }
 
@@ -67,9 +68,8 @@ constexpr int KNT = 256;
 // Generic fused vector kernel: op.elem() per element, then ND sums reduced and
 // handed to op.finish() in one block.
 template <int ND, class Op>
-__global__ void __launch_bounds__(KNT) k_vec(const Op op, long n3, int nblk, RedSlots rs, int* __restrict__ status) {
+__global__ void __launch_bounds__(KNT) k_vec(const Op op, long n3, int nblk, RedSlots rs, int* status) {
     const int rhs = blockIdx.y;
-    pdl_trigger();
     pdl_wait();
     if (status[rhs]) return;
     double2 acc[ND > 0 ? ND : 1];
@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(KNT) k_vec(const Op op, long n3, int nblk, Red
     for (int m = 0; m < (ND > 0 ? ND : 1); m++) acc[m] = make_double2(0, 0);
     const KState s = op.stt[rhs];
     for (long i = (long)blockIdx.x * KNT + threadIdx.x; i < n3; i += (long)nblk * KNT) op.elem(s, rhs, i, acc);
+    __syncthreads();  // the block's vectors are written: the next kernel may read them through ldg
+    pdl_trigger();
     if constexpr (ND > 0) {
         if (reduce_across_blocks<KNT, ND>(acc, rhs, blockIdx.x, nblk, rs) && threadIdx.x == 0)
             op.finish(rhs, op.stt[rhs], status[rhs], acc);

@@ -405,9 +405,9 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_fwd_x(const MvArgs<T> a,
     const int j0 = blockIdx.x * TL, k = blockIdx.y;
     const int nl = min(TL, ny - j0);
     load_twiddles<C, L, NT>(tw, a.twx);
-    pdl_trigger();
     pdl_wait();
-    if (a.status && __ldcg(a.status + rhs)) return;
+    pdl_trigger();
+    if (a.status && a.status[rhs]) return;
     using Src = FwdXLoad<T, TAB, Pre>;
     Src src{a.tab_of(rhs), a.alpha_of(rhs), a.amode, (int)a.nmax, nx, pre, k * nx * ny + j0 * nx, nl, TL};
     src.pre.bind(a, rhs);
@@ -451,9 +451,9 @@ __global__ void __launch_bounds__(TT::NTY, TT::MINBY) k_pass_y(const MvArgs<T> a
     const int XE = a.g.X / V, ny = a.g.ny, nz = a.g.nz;
     const int i0 = blockIdx.x * TL, k = blockIdx.y;
     load_twiddles<W, L, NT>(tw, a.twy);
-    pdl_trigger();
     pdl_wait();
-    if (a.status && __ldcg(a.status + rhs)) return;
+    pdl_trigger();
+    if (a.status && a.status[rhs]) return;
     const int nv = min(TL, XE - i0);
     E* b1 = reinterpret_cast<E*>(a.B1 + rhs * a.g.b1_rhs) + ((long)c * nz + k) * ny * XE + i0;
     E* b2 = reinterpret_cast<E*>(a.B2 + rhs * a.g.b2_rhs) + ((long)c * nz + k) * L * XE + i0;
@@ -587,7 +587,10 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
     const int nx = a.g.nx, ny = a.g.ny, nz = a.g.nz, Y = a.g.Y, XE = a.g.X / V;
     const int i0 = blockIdx.y * TL;
     const int qy = blockIdx.z;                    // 0 .. ny
-    if (hm && !(qy > 0 && qy < ny)) return;
+    if (hm && !(qy > 0 && qy < ny)) {
+        pdl_wait();
+        return;
+    }
     const int t0 = i0 * V / 2;           // first pair of the tile
     load_twiddles<W, L, NT>(tw, a.twz);
     // the tile's columns of the compressed spectrum (contiguous each) are
@@ -610,9 +613,9 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
         cp_async_commit();
     }
     // the spectrum and the twiddles are constant: only B2 waits for the y pass
-    pdl_trigger();
     pdl_wait();
-    if (a.status && __ldcg(a.status + rhs)) {
+    pdl_trigger();
+    if (a.status && a.status[rhs]) {
         if constexpr (!TT::ZSMALL) cp_async_wait_all();
         return;
     }
@@ -769,9 +772,8 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_inv_x(const MvArgs<T> a,
     const int j0 = blockIdx.x * TL, k = blockIdx.y;
     const int nl = min(TL, ny - j0);
     load_twiddles<C, L, NT>(tw, a.twx);
-    pdl_trigger();
     pdl_wait();
-    if (a.status && __ldcg(a.status + rhs)) return;
+    if (a.status && a.status[rhs]) return;
     const C* base = a.B1 + rhs * a.g.b1_rhs + ((long)k * ny + j0) * L;
     InvXStore<T, TAB, Epi> dst{a.tab_of(rhs), a.b + rhs * a.xstride, a.y + rhs * a.xstride, a.inv_m, nx,
                                k * nx * ny + j0 * nx, nl, TL, epi};
@@ -788,6 +790,8 @@ __global__ void __launch_bounds__(TT::NTX, TT::MINBX) k_inv_x(const MvArgs<T> a,
     if constexpr (TT::NPX > 1)
         stockham_range<C, L, NB, NT, -1, typename TT::LayX, true, TT::NPX, 1, TT::RX, SmemIO, InvXStore<T, TAB, Epi>,
                        PLAN_X>(sm, tw, SmemIO{}, dst);
+    __syncthreads();  // the block's part of y is written: the next kernel may read it through ldg
+    pdl_trigger();
     if constexpr (Epi::ND > 0) {
         double2 tot[Epi::ND + Epi::NDP];
         if (reduce_rows<NT, Epi::ND, Epi::NDP>(dst.epi.acc, tot, rhs, blockIdx.x, k, gridDim.x, gridDim.y, red) &&
