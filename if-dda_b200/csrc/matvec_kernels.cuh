@@ -105,9 +105,13 @@ template <class T> struct MvArgs {
 //    or more, three were slower (FP64 at 64^3 57.9 against 45.2 us: the extra
 //    round trip through shared memory).
 // Register caps of the y passes and of zconv's small middles (RK up to 5): 102
-// (five warps per quarter SM; 84 for first radices up to 8) instead of 128:
-// 12 right-hand sides of 48x40x32 in FP64 5.51 -> 5.24 ms a solve, 75x45x29 x2
-// 86.7 -> 84.9 us a mat-vec.
+// (five warps per quarter SM) instead of 128: 12 right-hand sides of 48x40x32
+// in FP64 5.51 -> 5.24 ms a solve, 75x45x29 x2 86.7 -> 84.9 us a mat-vec.  First
+// radices up to 8 take 84 where the middle has up to 4 points (128x128x16 x2
+// 183.7 us in FP64 against 187.4 at 102 and 193.5 at 128); with 5 points (z
+// lengths 10, 20, 40) that spills 170 to 460 bytes a thread, and 102 (none in
+// FP64, up to 32 in FP32) is faster: 128x128x20 120.5 -> 118.3 us (128: 124.3),
+// in FP32 63.3 -> 60.2 (62.2), 256x256x5 in FP32 98.0 -> 95.2 (103.4).
 // The variants are compiled for lengths of 64 and more; the tile chooser
 // (tune_tiles) times both on the caller's grid and keeps one per grid.  The
 // two agree to rounding.
@@ -202,7 +206,7 @@ template <class T, int L, int V = 0> struct MvTiles {
     using LayZ = Layout<NBZ, 1, true, zpadsh(TLZ), zpadoff(TLZ)>;
     static constexpr int MINBX = minblocks(NTX, S == 8 ? 80 : (RX > 8 ? 128 : 102));
     static constexpr int MINBY = minblocks(NTY, RY == 32 ? 168 : 102);
-    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : (RZ == 16 ? 102 : 84)));
+    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : (RZ == 16 || RK == 5 ? 102 : 84)));
     static constexpr size_t smem_x = (size_t)L * S + (size_t)NBX * LP * S;
     static constexpr size_t smem_y = (size_t)L * S + (size_t)L * NBY * SE;
     static constexpr size_t smem_z = zbytes(TLZ);
