@@ -512,15 +512,25 @@ __device__ __forceinline__ cpair gfma2(cpair acc, float2 g0, float2 g1, float s,
                  fma2(gx, v.im, fma2(gy, v.re, acc.im))};
 }
 
+// v with its sign bits flipped where f is the sign bit (0: v)
+__device__ __forceinline__ float2 flip(float2 v, unsigned f) {
+    return make_float2(__uint_as_float(__float_as_uint(v.x) ^ f), __uint_as_float(__float_as_uint(v.y) ^ f));
+}
+__device__ __forceinline__ double2 flip(double2 v, unsigned f) {
+    return make_double2(__hiloint2double(__double2hiint(v.x) ^ (int)f, __double2loint(v.x)),
+                        __hiloint2double(__double2hiint(v.y) ^ (int)f, __double2loint(v.y)));
+}
+
 // v <- G v for the RK points j + r NJ of one column; g: its slice [c6][qz].
-// Spectral mirrors: z beyond nz flips xz and yz, MY (row Y - qy) xy and yz
+// Spectral mirrors: z beyond nz flips xz and yz, the row Y - qy xy and yz
 // (component x of a mirrored column is stored negated, so xy and xz need no
-// flip for X - qx).
-template <class E, int L, int RK, bool MY, class W>
-__device__ __forceinline__ void zmultiply(E (&v)[3][RK], const W* g, int j) {
+// flip for X - qx).  MY: the row is a mirrored one (1), is not (0), or is where
+// my is the sign bit (-1).
+template <class E, int L, int RK, int MY, class W>
+__device__ __forceinline__ void zmultiply(E (&v)[3][RK], const W* g, unsigned my, int j) {
     using T = typename elem_traits<E>::T;
     constexpr int NJ = L / RK, NQ = L / 2 + 1;
-    const T sy = MY ? T(-1) : T(1);
+    const T sy = MY == 1 ? T(-1) : T(1);
 #pragma unroll
     for (int r = 0; r < RK; r++) {
         const int p = j + r * NJ;
@@ -529,15 +539,17 @@ __device__ __forceinline__ void zmultiply(E (&v)[3][RK], const W* g, int j) {
         const W* gq = g + (mir ? L - p : p);
         const T sz = mir ? T(-1) : T(1);
         const E x = v[0][r], y = v[1][r], z = v[2][r];
-        const W gxy = gq[NQ], gxz = gq[2 * NQ], gyz = gq[4 * NQ];
+        const W gxy = MY < 0 ? flip(gq[NQ], my) : gq[NQ], gxz = gq[2 * NQ];
+        const W gyz = MY < 0 ? flip(gq[4 * NQ], my) : gq[4 * NQ];
         v[0][r] = gfma(gfma(gmul(gq[0], x), gxy, sy, y), gxz, sz, z);
         v[1][r] = gfma(gfma(gmul(gq[3 * NQ], y), gxy, sy, x), gyz, sy * sz, z);
         v[2][r] = gfma(gfma(gmul(gq[5 * NQ], z), gxz, sz, x), gyz, sy * sz, y);
     }
 }
-// the FP32 pair t = 0, whose two values have columns of their own
+// the same for an FP32 pair whose two values have columns of their own (t = 0)
 template <int L, int RK>
-__device__ __forceinline__ void zmultiply_ends(cpair (&v)[3][RK], const float2* g0, const float2* g1, float sy, int j) {
+__device__ __forceinline__ void zmultiply_ends(cpair (&v)[3][RK], const float2* g0, const float2* g1, unsigned my,
+                                               int j) {
     constexpr int NJ = L / RK, NQ = L / 2 + 1;
 #pragma unroll
     for (int r = 0; r < RK; r++) {
@@ -547,12 +559,12 @@ __device__ __forceinline__ void zmultiply_ends(cpair (&v)[3][RK], const float2* 
         const float sz = mir ? -1.f : 1.f;
         const cpair x = v[0][r], y = v[1][r], z = v[2][r];
         const cpair o = czero<cpair>();
-        v[0][r] = gfma2(gfma2(gfma2(o, g0[q], g1[q], 1.f, x), g0[q + NQ], g1[q + NQ], sy, y), g0[q + 2 * NQ],
-                        g1[q + 2 * NQ], sz, z);
-        v[1][r] = gfma2(gfma2(gfma2(o, g0[q + 3 * NQ], g1[q + 3 * NQ], 1.f, y), g0[q + NQ], g1[q + NQ], sy, x),
-                        g0[q + 4 * NQ], g1[q + 4 * NQ], sy * sz, z);
+        const float2 xy0 = flip(g0[q + NQ], my), xy1 = flip(g1[q + NQ], my);
+        const float2 yz0 = flip(g0[q + 4 * NQ], my), yz1 = flip(g1[q + 4 * NQ], my);
+        v[0][r] = gfma2(gfma2(gfma2(o, g0[q], g1[q], 1.f, x), xy0, xy1, 1.f, y), g0[q + 2 * NQ], g1[q + 2 * NQ], sz, z);
+        v[1][r] = gfma2(gfma2(gfma2(o, g0[q + 3 * NQ], g1[q + 3 * NQ], 1.f, y), xy0, xy1, 1.f, x), yz0, yz1, sz, z);
         v[2][r] = gfma2(gfma2(gfma2(o, g0[q + 5 * NQ], g1[q + 5 * NQ], 1.f, z), g0[q + 2 * NQ], g1[q + 2 * NQ], sz, x),
-                        g0[q + 4 * NQ], g1[q + 4 * NQ], sy * sz, y);
+                        yz0, yz1, sz, y);
     }
 }
 
@@ -639,6 +651,7 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
         cp_async_wait_all();
         __syncthreads();
     }
+    const unsigned my = hm ? 0x80000000u : 0u;
     // ---- fused middle: read, transform, multiply, transform (registers) ----
     E v[PERM][3][RK];
 #pragma unroll
@@ -672,15 +685,20 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
             const bool ends = V == 2 ? t0 + t == 0 : (t0 == 0 && il == 1);
             if constexpr (V == 2) {
                 const W* g0 = TT::ZSMALL ? gbase + (long)(t0 + t) * (6 * TT::NQ) : gs + t * GST;
-                if (ends)
-                    zmultiply_ends<L, RK>(v[q], g0, TT::ZSMALL ? gbase + (long)nx * (6 * TT::NQ) : gs + TC * GST,
-                                          hm ? -1.f : 1.f, j);
-                else if (hm) zmultiply<E, L, RK, true>(v[q], g0, j);
-                else zmultiply<E, L, RK, false>(v[q], g0, j);
+                // The whole tile of t = 0 takes the form with two columns, and the row's sign is a
+                // value: no warp runs two forms, and the code, which a small grid's few waves
+                // fetch about as often as they run it, is shorter (zconv of 16^3 x8 4.28 -> 3.74 us,
+                // 64^3 20.9 -> 19.9).  FP64, whose columns are one each, keeps a form per row sign
+                // (35.2 against 35.7 us at 64^3).
+                if (t0 == 0)
+                    zmultiply_ends<L, RK>(v[q], g0,
+                                          !ends ? g0 : TT::ZSMALL ? gbase + (long)nx * (6 * TT::NQ) : gs + TC * GST, my,
+                                          j);
+                else zmultiply<E, L, RK, -1>(v[q], g0, my, j);
             } else {
                 const W* gcol = TT::ZSMALL ? gbase + (long)(ends ? nx : t0 + t) * (6 * TT::NQ) : gs + (ends ? TC : t) * GST;
-                if (hm) zmultiply<E, L, RK, true>(v[q], gcol, j);
-                else zmultiply<E, L, RK, false>(v[q], gcol, j);
+                if (hm) zmultiply<E, L, RK, 1>(v[q], gcol, my, j);
+                else zmultiply<E, L, RK, 0>(v[q], gcol, my, j);
             }
         }
         // inverse pass 0 of the reversed plan: Ns = 1, inputs j + r NJ, no twiddles
