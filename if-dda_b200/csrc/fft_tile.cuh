@@ -66,9 +66,12 @@ __host__ __device__ constexpr bool has_dft(int r) {
     return r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 8 || r == 10 || r == 12 || r == 16 || r == 32;
 }
 // Plans of the mat-vec passes (policy 0 is the general rule above):
-//  PLAN_Z: two passes up to 384, the second (whose butterflies hold all three
-//      components of a column in registers) of at most 8 points up to 256 and
-//      12 above: 16-byte elements at three times 8 points take 96 registers;
+//  PLAN_Z: one pass up to 8, two up to 384, the second (whose butterflies hold
+//      all three components of a column in registers) of at most 8 points up
+//      to 256 and 12 above: 16-byte elements at three times 8 points take 96
+//      registers.  Factors 5 go into the first pass: with a five-point middle
+//      zconv of 256x256x5 took 103 us in FP64 instead of 40 (46.5, 22.4 in
+//      FP32), of 128x128x20 43.3 instead of 37.7 (22.3, 19.9);
 //  PLAN_Z3: three passes with small radices: one shared-memory round trip more
 //      per direction, for half the registers and twice the warps;
 //  PLAN_Y: two passes up to 512;
@@ -82,16 +85,16 @@ __host__ __device__ constexpr RadixPlan plan_table(int L, int policy) {
     switch (policy) {
     case PLAN_Z:
         switch (L) {
-        case 4: return {{2, 2}};
-        case 6: return {{2, 3}};
-        case 8: return {{4, 2}};
-        case 10: return {{2, 5}};
+        case 4: return {{4}};
+        case 6: return {{6}};
+        case 8: return {{8}};
+        case 10: return {{5, 2}};
         case 12: return {{4, 3}};
         case 16: return {{4, 4}};
-        case 20: return {{4, 5}};
+        case 20: return {{10, 2}};
         case 24: return {{8, 3}};
         case 32: return {{8, 4}};
-        case 40: return {{8, 5}};
+        case 40: return {{10, 4}};
         case 48: return {{16, 3}};
         case 64: return {{16, 4}};
         case 80: return {{16, 5}};

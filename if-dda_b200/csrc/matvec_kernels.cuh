@@ -94,7 +94,10 @@ template <class T> struct MvArgs {
 //    once, and the solver's passes took 24.9 instead of 18.5 us;
 //  * y passes: 16 columns of 16 bytes from length 64 on, 8 below and for V = 1
 //    (FP64 there and back at 64^3 34.5 against 36.6 us; 8 leave a small
-//    lattice more blocks);
+//    lattice more blocks).  Up to length 16 a column is one thread's: 16
+//    columns (8 x 8 x 8, 8 right-hand sides: 8.6 us a product against 9.0 with
+//    8 and 9.2 with 32), and 32 up to length 8 (64 x 2 x 64 in FP64 17.8 us
+//    with 8, 14.6 with 16, 13.2 with 32);
 //  * zconv: 8 columns of 16 bytes, rows of 128 bytes.  4 columns (V = 1 below
 //    160) and 2 give more and smaller blocks, but their narrower rows cost more
 //    than that: FP64 at 64^3 43.5, 47.5 and 65 us, FP32 27.9, 29.5 and 40.5 us.
@@ -104,14 +107,19 @@ template <class T> struct MvArgs {
 //    fit: FP32 at 192^3 1.21 -> 0.89 ms.  Below, where two passes leave 12 warps
 //    or more, three were slower (FP64 at 64^3 57.9 against 45.2 us: the extra
 //    round trip through shared memory).
+//    Up to length 8 a column is one thread's, with no shared memory in
+//    between, and a block takes 32 columns (64 at length 2), at length 10 16:
+//    with 8 columns and two passes most threads had no work.  Product of
+//    256x256x1 in FP64 66.1 -> 33.7 us, 128x128x2 x4 70.4 -> 44.9, 128x128x4 x2
+//    55.2 -> 43.8, 256x256x5 192.7 -> 130.9; in FP32 37.5 -> 25.0, 42.4 -> 31.2,
+//    33.9 -> 30.9, 97.4 -> 67.0.
 // Register caps of the y passes and of zconv's small middles (RK up to 5): 102
-// (five warps per quarter SM) instead of 128: 12 right-hand sides of 48x40x32
-// in FP64 5.51 -> 5.24 ms a solve, 75x45x29 x2 86.7 -> 84.9 us a mat-vec.  First
-// radices up to 8 take 84 where the middle has up to 4 points (128x128x16 x2
-// 183.7 us in FP64 against 187.4 at 102 and 193.5 at 128); with 5 points (z
-// lengths 10, 20, 40) that spills 170 to 460 bytes a thread, and 102 (none in
-// FP64, up to 32 in FP32) is faster: 128x128x20 120.5 -> 118.3 us (128: 124.3),
-// in FP32 63.3 -> 60.2 (62.2), 256x256x5 in FP32 98.0 -> 95.2 (103.4).
+// (five warps per quarter SM; 84 for first radices up to 8 and at length 20)
+// instead of 128: 12 right-hand sides of 48x40x32 in FP64 5.51 -> 5.24 ms a
+// solve, 75x45x29 x2 86.7 -> 84.9 us a mat-vec; 128x128x16 x2 183.7 us a mat-vec
+// in FP64 with 84, 187.4 with 102 and 193.5 with 128; 40x40x20 20.2 us with 84,
+// 19.3 with 102, x8 76.7 and 77.6.  One pass takes what three times L points
+// need (128x128x2 x4 in FP64 45.9 us with 84, which spills, 42.8 with 102 or 128).
 // The variants are compiled for lengths of 64 and more; the tile chooser
 // (tune_tiles) times both on the caller's grid and keeps one per grid.  The
 // two agree to rounding.
@@ -127,7 +135,7 @@ template <class T, int L, int V = 0> struct MvTiles {
     static constexpr int SE = (int)sizeof(E);
     static constexpr int SMEM_X = L >= 64 ? 16384 : 8192;
     static constexpr int TLX = clamp_pow2(SMEM_X / (3 * (L + 1) * S), 1, 16);
-    static constexpr int TLY = V == 0 && L >= 64 ? 16 : 8;
+    static constexpr int TLY = L <= 8 ? 32 : L <= 16 || (V == 0 && L >= 64) ? 16 : 8;
     static constexpr int NBX = 3 * TLX, NBY = TLY;
     // x tile: points contiguous with one pad word every 16, line pitch = 8 (mod 16)
     static constexpr int lpitch() {
@@ -191,13 +199,13 @@ template <class T, int L, int V = 0> struct MvTiles {
         return (size_t)L * S + (size_t)zspan(tl) * 3 * tl * SE + (ZSMALL ? 0 : (size_t)(gcols(tl) + 1) * GST * S);
     }
     static constexpr int ztile() {
-        int tl = V == 1 && !ZSMALL ? 4 : 8;
+        int tl = NPZ == 1 ? (L == 2 ? 64 : 32) : L == 10 ? 16 : V == 1 && !ZSMALL ? 4 : 8;
         while (tl > 2 && zbytes(tl) > 112 * 1024) tl /= 2;
         return tl;
     }
     static constexpr int TLZ = ztile(), NBZ = 3 * TLZ, TCZ = gcols(TLZ);
     static_assert(TLZ >= 2, "a zconv tile holds whole pairs");
-    static constexpr int NTZ = ZSMALL ? round32(TLZ * NJZ, 512) : round32(NBZ * (L / RZ) > TLZ * NJZ ? NBZ * (L / RZ) : TLZ * NJZ, 512);
+    static constexpr int NTZ = ZSMALL || NPZ == 1 ? round32(TLZ * NJZ, 512) : round32(NBZ * (L / RZ) > TLZ * NJZ ? NBZ * (L / RZ) : TLZ * NJZ, 512);
     // L2 prefetch size of the column reads of zconv and the y passes (rows of
     // 32 to 256 bytes that neighbouring blocks read at the same time)
     static constexpr int ZPF = 256;
@@ -206,7 +214,7 @@ template <class T, int L, int V = 0> struct MvTiles {
     using LayZ = Layout<NBZ, 1, true, zpadsh(TLZ), zpadoff(TLZ)>;
     static constexpr int MINBX = minblocks(NTX, S == 8 ? 80 : (RX > 8 ? 128 : 102));
     static constexpr int MINBY = minblocks(NTY, RY == 32 ? 168 : 102);
-    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : (RZ == 16 || RK == 5 ? 102 : 84)));
+    static constexpr int MINBZ = minblocks(NTZ, ZSMALL ? 84 : NPZ == 1 ? (L == 2 ? 84 : L == 4 ? 128 : L == 6 ? 168 : 248) : RK >= 10 ? 248 : (RZ == 32 || RK > 5 ? 168 : (RZ == 16 || L == 40 ? 102 : 84)));
     static constexpr size_t smem_x = (size_t)L * S + (size_t)NBX * LP * S;
     static constexpr size_t smem_y = (size_t)L * S + (size_t)L * NBY * SE;
     static constexpr size_t smem_z = zbytes(TLZ);
@@ -616,15 +624,25 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
     if constexpr (!TT::ZSMALL) {
         constexpr int CH = 6 * TT::NQ * (int)sizeof(W) / 16;
         static_assert(6 * TT::NQ * sizeof(W) % 16 == 0 && GST * sizeof(W) % 16 == 0, "16-byte copies");
+        const char* src = reinterpret_cast<const char*>(gbase + (long)t0 * (6 * TT::NQ));
+        char* dst = reinterpret_cast<char*>(gs);
+        if constexpr (CH < NT) {  // several columns at a time
+            for (int e = threadIdx.x; e < min(TC, nx - t0) * CH; e += NT)
+                cp_async16(dst + e / CH * (GST * (int)sizeof(W)) + e % CH * 16, src + 16 * e);
+            if (t0 == 0 && (int)threadIdx.x < CH)
+                cp_async16(dst + TC * (GST * (int)sizeof(W)) + 16 * threadIdx.x,
+                           src + (long)nx * (CH * 16) + 16 * threadIdx.x);
+        } else {
 #pragma unroll
-        for (int col = 0; col <= TC; col++) {
-            const int qx = col < TC ? t0 + col : nx;
-            if (!(col < TC ? qx < nx : t0 == 0)) continue;
-            const char* src = reinterpret_cast<const char*>(gbase + (long)qx * (6 * TT::NQ)) + 16 * threadIdx.x;
-            char* dst = reinterpret_cast<char*>(gs + col * GST) + 16 * threadIdx.x;
+            for (int col = 0; col <= TC; col++) {
+                const int qx = col < TC ? t0 + col : nx;
+                if (!(col < TC ? qx < nx : t0 == 0)) continue;
+                const char* cs = src + (long)(qx - t0) * (CH * 16) + 16 * threadIdx.x;
+                char* cd = dst + col * (GST * (int)sizeof(W)) + 16 * threadIdx.x;
 #pragma unroll
-            for (int ch = 0; ch < CH; ch += NT)
-                if (ch + NT <= CH || ch + (int)threadIdx.x < CH) cp_async16(dst + 16 * ch, src + 16 * ch);
+                for (int ch = 0; ch < CH; ch += NT)
+                    if (ch + NT <= CH || ch + (int)threadIdx.x < CH) cp_async16(cd + 16 * ch, cs + 16 * ch);
+            }
         }
         cp_async_commit();
     }
@@ -666,7 +684,8 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
             for (int r = 0; r < RK; r++) {
                 const int p = j + r * NJ;
                 if constexpr (NP == 1) {
-                    v[q][c][r] = (2 * p >= L) ? czero<E>() : zload.template load<E>(b, p);
+                    // (no load for a column beyond the last: the one before is being written)
+                    v[q][c][r] = 2 * p >= L || il >= nv ? czero<E>() : zload.template load<E>(b, p);
                 } else if constexpr (read_split<LZ>(NJ, RK)) {
                     v[q][c][r] = sm[LZ::addr(j, b) + LZ::pidx(r * NJ) * LZ::PS];
                 } else {
