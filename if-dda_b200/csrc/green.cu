@@ -94,10 +94,11 @@ static void launch_gyz(const GreenGeom& gg, const double2* src, double2* d64, fl
                        cudaStream_t st) {
     using TT = GreenTiles<L>;
     const int W = gg.nx + 1;
-    dim3 grid((W + TT::TLY - 1) / TT::TLY, AXIS == 1 ? gg.nz + 1 : gg.ny + 1, 6);
-    ensure_smem(k_green_yz<L, AXIS>, TT::smem_y);
+    const unsigned tiles = (W + TT::tl(AXIS) - 1) / TT::tl(AXIS);
+    const dim3 grid = AXIS == 1 ? dim3(tiles, gg.nz + 1, 6) : dim3(6, tiles, gg.ny + 1);
+    ensure_smem(k_green_yz<L, AXIS>, TT::smem_yz(AXIS));
     count_launch();
-    k_green_yz<L, AXIS><<<grid, TT::NT, TT::smem_y, st>>>(gg, src, d64, d32, tw);
+    k_green_yz<L, AXIS><<<grid, TT::NT, TT::smem_yz(AXIS), st>>>(gg, src, d64, d32, tw);
 }
 
 // smallest n' >= n with 2 n' a compiled FFT length (n itself when none is)

@@ -40,9 +40,13 @@ template <int L> struct GreenTiles {
     static constexpr int NT = 256;
     static constexpr int LSX = (6 * TLX) | 1;
     static constexpr size_t smem_x = (size_t)L * S + (size_t)L * LSX * S;
-    // one column of padding: the z pass reads its lines point by point
-    static constexpr int LSY = TLY + 1;
-    static constexpr size_t smem_y = (size_t)L * S + (size_t)L * LSY * S;
+    // Columns of a block of the y and of the z pass: 32 in the z pass up to
+    // length 48 (16: 256x256x5 163 us instead of 147).  The z pass, which reads
+    // its lines point by point to write them, has one column of padding; the y
+    // pass has none (with it the spectrum of 64x80x64 took 147 us instead of 128).
+    static constexpr int tl(int axis) { return axis == 1 || L > 48 ? TLY : clamp_pow2(49152 / (L * S), 2, 32); }
+    static constexpr int ls(int axis) { return axis == 1 ? tl(1) : tl(2) + 1; }
+    static constexpr size_t smem_yz(int axis) { return (size_t)L * S + (size_t)L * ls(axis) * S; }
 };
 
 // T_ab(r), the six independent components xx, xy, xz, yy, yz, zz
@@ -209,15 +213,17 @@ __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_yz(const GreenGeom 
                                                                 const double2* __restrict__ tw_axis) {
     using C = double2;
     using TT = GreenTiles<L>;
-    constexpr int TL = TT::TLY, LS = TT::LSY, NT = TT::NT;
+    constexpr int TL = TT::tl(AXIS), LS = TT::ls(AXIS), NT = TT::NT;
     extern __shared__ __align__(16) unsigned char raw[];
     C* tw = reinterpret_cast<C*>(raw);
     C* sm = tw + L;
     const int W = g.nx + 1;
-    const int q0 = blockIdx.x * TL, c = blockIdx.z;
+    // AXIS 1: o = kk (0..nz), lines along y;  AXIS 2: o = qy (0..ny), lines along z, the components fastest in the
+    // grid: their lines lie side by side, so the memory's sectors and lines that they share are written together
+    // (with the component slowest 256x256x20 took 486 us)
+    const int q0 = (AXIS == 1 ? blockIdx.x : blockIdx.y) * TL;
+    const int o = AXIS == 1 ? blockIdx.y : blockIdx.z, c = AXIS == 1 ? blockIdx.z : blockIdx.x;
     load_twiddles<C, L, NT>(tw, tw_axis);
-    // AXIS 1: blockIdx.y = kk (0..nz), lines along y;  AXIS 2: blockIdx.y = qy (0..ny), lines along z
-    const int o = blockIdx.y;
     const int keep = AXIS == 1 ? g.ny + 1 : g.nz + 1;
     const int half = AXIS == 1 ? g.ny : g.nz;
     const double sgn = AXIS == 1 ? green_py(c) : green_pz(c);
@@ -247,11 +253,12 @@ __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_yz(const GreenGeom 
             const int p = e / TL, il = e - p * TL;
             if (q0 + il < W) put(p, il, (((long)c * (g.nz + 1) + o) * (g.ny + 1) + p) * W + q0 + il);
         }
-    } else {  // a warp writes one line: z is contiguous
-        for (int il = threadIdx.x / 32; il < TL; il += NT / 32) {
-            if (q0 + il >= W) break;
-            const long line = (((long)o * W + q0 + il) * 6 + c) * (g.nz + 1);
-            for (int p = threadIdx.x & 31; p < keep; p += 32) put(p, il, line + p);
+    } else {  // z is contiguous: consecutive threads write a line, and the next one where it is short
+        constexpr int KEEP = L / 2 + 1;
+        const long line = ((long)o * W + q0) * 6 + c;
+        for (int e = threadIdx.x; e < TL * KEEP; e += NT) {
+            const int il = e / KEEP, p = e - il * KEEP;
+            if (q0 + il < W) put(p, il, (line + 6 * il) * KEEP + p);
         }
     }
 }
