@@ -104,27 +104,29 @@ __device__ __forceinline__ void ydft_plane(const MicGeom& m, const double2* __re
 // One pupil point reads nz ny values of Q one after the other, and there are
 // only nb S^2 points (1690 for 10 illuminations of a 24^3 object: 7 blocks of
 // one thread per point took 319 us, latency of a serial chain).  So a block
-// takes FAR_P points and cuts their planes into FAR_G shares, summed in order
-// at the end.
-constexpr int FAR_P = 16, FAR_G = 16;
-// adds the FAR_G shares of each of a block's points in order, into thread g = 0's acc
-template <int N> __device__ __forceinline__ void far_sum(double2 (&acc)[N], int p, int g) {
-    __shared__ double2 part[FAR_G][FAR_P][N];
+// cuts the planes of its points into G shares, summed in order at the end.
+constexpr int FAR_NT = 256;
+// adds the G shares of each of a block's points in order, into thread g = 0's acc
+template <int G, int N> __device__ __forceinline__ void far_sum(double2 (&acc)[N], int p, int g) {
+    if constexpr (G == 1) return;
+    __shared__ double2 part[G][FAR_NT / G][N];
 #pragma unroll
     for (int c = 0; c < N; c++) part[g][p][c] = acc[c];
     __syncthreads();
     if (g > 0) return;
-    for (int h = 1; h < FAR_G; h++)
+    for (int h = 1; h < G; h++)
 #pragma unroll
         for (int c = 0; c < N; c++) acc[c] = cadd(acc[c], part[h][p][c]);
 }
-__global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far(const MicGeom m, int nb, const double2* __restrict__ Q,
+template <int G>
+__global__ void __launch_bounds__(FAR_NT) k_mic_far(const MicGeom m, int nb, const double2* __restrict__ Q,
                                                             const double* __restrict__ zplane,
                                                             const double2* __restrict__ tw, double2* __restrict__ Ed) {
     const int S = m.S();
     const long total = (long)nb * S * S;
-    const int p = threadIdx.x % FAR_P, g = threadIdx.x / FAR_P;
-    const long t = (long)blockIdx.x * FAR_P + p;
+    constexpr int P = FAR_NT / G;
+    const int p = threadIdx.x % P, g = threadIdx.x / P;
+    const long t = (long)blockIdx.x * P + p;
     const int irow = (int)(t % S);
     const int jrow = (int)((t / S) % S);
     const int b = (int)(t / ((long)S * S));
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far(const MicGeom m, int 
         const double2 exy = make_double2(cs, sn);
         const double2 den = make_double2(0.0, -2.0 * 3.14159265358979323846 * kz);
         const int step = posmod(j, n), ph0 = posmod((long)j * (-(n / 2)), n);
-        for (int k = g * m.nz / FAR_G; k < (g + 1) * m.nz / FAR_G; k++) {
+        for (int k = g * m.nz / G; k < (g + 1) * m.nz / G; k++) {
             double2 p0, p1, p2;
             ydft_plane(m, Q, tw, b, k, irow, ph0, step, p0, p1, p2);
             // ctmp = (kx P_x + ky P_y + kz dside P_z) / k0, on the side dside
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far(const MicGeom m, int 
 #pragma unroll
         for (int c = 0; c < 3; c++) o[c] = cscale(o[c], k02);
     }
-    far_sum<3>(o, p, g);
+    far_sum<G, 3>(o, p, g);
     if (g > 0 || t >= total) return;
     double2* e = Ed + t * 3;
 #pragma unroll
@@ -167,13 +169,15 @@ __global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far(const MicGeom m, int 
 //   E+_c = sum_k (P_c - k+_c (k+.P) / k0^2) exp(-i kz z_k) exp(-i (var1 i + var2 j))
 //   E-_c = sum_k (P_c - k-_c (k-.P) / k0^2) exp(+i kz z_k) exp(-i (var1 i + var2 j))
 // with k+- = (kx, ky, +-kz); Ed holds E+ for all nb, then E-.
-__global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far2(const MicGeom m, int nb, const double2* __restrict__ Q,
+template <int G>
+__global__ void __launch_bounds__(FAR_NT) k_mic_far2(const MicGeom m, int nb, const double2* __restrict__ Q,
                                                              const double* __restrict__ zplane,
                                                              const double2* __restrict__ tw, double2* __restrict__ Ed) {
     const int S = m.S();
     const long total = (long)nb * S * S;
-    const int p = threadIdx.x % FAR_P, g = threadIdx.x / FAR_P;
-    const long t = (long)blockIdx.x * FAR_P + p;
+    constexpr int P = FAR_NT / G;
+    const int p = threadIdx.x % P, g = threadIdx.x / P;
+    const long t = (long)blockIdx.x * P + p;
     const int irow = (int)(t % S);
     const int jrow = (int)((t / S) % S);
     const int b = (int)(t / ((long)S * S));
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far2(const MicGeom m, int
         sincos(-__dadd_rn(__dmul_rn(m.var1, (double)i), __dmul_rn(m.var2, (double)j)), &sn, &cs);
         const double2 exy = make_double2(cs, sn);
         const int step = posmod(j, n), ph0 = posmod((long)j * (-(n / 2)), n);
-        for (int k = g * m.nz / FAR_G; k < (g + 1) * m.nz / FAR_G; k++) {
+        for (int k = g * m.nz / G; k < (g + 1) * m.nz / G; k++) {
             double2 p0, p1, p2;
             ydft_plane(m, Q, tw, b, k, irow, ph0, step, p0, p1, p2);
             sincos(kz * zplane[k], &sn, &cs);
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(FAR_P * FAR_G) k_mic_far2(const MicGeom m, int
             o[5] = cadd(o[5], cmul(cadd(p2, make_double2(kz * tn.x / m.k0, kz * tn.y / m.k0)), dn));
         }
     }
-    far_sum<6>(o, p, g);
+    far_sum<G, 6>(o, p, g);
     if (g > 0 || t >= total) return;
     double2* e = Ed + t * 3;
     double2* f = e + (long)nb * S * S * 3;
@@ -590,6 +594,15 @@ template <int L> void launch_image(const MicGeom& m, int nb, const double2* F, c
     IFDDA_CUDA(cudaGetLastError());
 }
 
+template <int G>
+void far_launch(const MicGeom& m, int nb, long ne, const double2* Q, const double* zplane, const double2* tw,
+                double2* Ed, cudaStream_t st, bool both_sides) {
+    constexpr int P = FAR_NT / G;
+    const unsigned blocks = (unsigned)((ne + P - 1) / P);
+    if (both_sides) k_mic_far2<G><<<blocks, FAR_NT, 0, st>>>(m, nb, Q, zplane, tw, Ed);
+    else k_mic_far<G><<<blocks, FAR_NT, 0, st>>>(m, nb, Q, zplane, tw, Ed);
+}
+
 }  // namespace
 
 bool image_length_supported(int n) {
@@ -610,8 +623,13 @@ void mic_farfield_dev(const MicGeom& m, int nb, const double2* FF, const double*
     k_mic_xdft<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(m, nb, FF, tw, Q);
     IFDDA_CUDA(cudaGetLastError());
     count_launch();
-    if (both_sides) k_mic_far2<<<(unsigned)((ne + FAR_P - 1) / FAR_P), FAR_P * FAR_G, 0, st>>>(m, nb, Q, zplane, tw, Ed);
-    else k_mic_far<<<(unsigned)((ne + FAR_P - 1) / FAR_P), FAR_P * FAR_G, 0, st>>>(m, nb, Q, zplane, tw, Ed);
+    switch (far_shares(m.nz, m.S())) {
+        case 1: far_launch<1>(m, nb, ne, Q, zplane, tw, Ed, st, both_sides); break;
+        case 2: far_launch<2>(m, nb, ne, Q, zplane, tw, Ed, st, both_sides); break;
+        case 4: far_launch<4>(m, nb, ne, Q, zplane, tw, Ed, st, both_sides); break;
+        case 8: far_launch<8>(m, nb, ne, Q, zplane, tw, Ed, st, both_sides); break;
+        default: far_launch<16>(m, nb, ne, Q, zplane, tw, Ed, st, both_sides); break;
+    }
     IFDDA_CUDA(cudaGetLastError());
 }
 

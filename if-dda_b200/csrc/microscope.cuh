@@ -30,6 +30,21 @@ struct MicGeom {
     __host__ __device__ int S() const { return 2 * imax + 1; }
 };
 
+// Shares that the far field cuts the planes of a pupil point into (a power of
+// two; the point's threads, 16 at most): no more than there are planes, so that
+// every thread has one, and no more than fill the GPU from the S^2 points of
+// one incidence.  One thread per point leaves small pupils to a serial chain (13^2
+// points of a 24^3 object, 10 incidences: 253 us, 38 with 16 shares), 16 are
+// mostly idle on thin objects and crowd large pupils (401^2 points of 64x64x1:
+// 670 us, 82 with one; 121^2 of 64x64x5: 105, 71 with 8).
+__host__ __device__ constexpr int far_shares(int nz, int S) {
+    int g = 16;
+    while (g > 1 && (g >= 2 * nz || (long)S * S * g > (1L << 17))) g /= 2;
+    return g;
+}
+static_assert(far_shares(1, 13) == 1 && far_shares(3, 13) == 4 && far_shares(24, 13) == 16, "planes");
+static_assert(far_shares(24, 121) == 8 && far_shares(24, 401) == 1 && far_shares(24, 4097) == 1, "points");
+
 // Far field Ed (nb x S x S x 3, entry ((b S + jrow) S + irow) 3 + c) of the
 // dipole moments FF (nb vectors of 3 nx ny nz, full box).  zplane: z of each
 // lattice plane; tw: exp(+2 pi i m / n), m < n; Q: nb nz ny S 3 scratch.
