@@ -54,11 +54,6 @@ template <class C> __host__ __device__ __forceinline__ C cmulc(C a, C b) {
 }
 template <class C, class S> __host__ __device__ __forceinline__ C cscale(C a, S s) { return mk(a.x * s, a.y * s); }
 template <class C> __host__ __device__ __forceinline__ C cconj(C a) { return mk(a.x, -a.y); }
-// multiply by (sign * i)
-template <int SIGN, class C> __host__ __device__ __forceinline__ C cmul_i(C a) {
-    return SIGN > 0 ? mk(-a.y, a.x) : mk(a.y, -a.x);
-}
-
 // Two complex FP32 values, real parts and imaginary parts together: the
 // element of the mat-vec's y and z passes in FP32.  Sums and products by
 // constants of both values are one packed instruction (add / mul / fma

@@ -213,20 +213,6 @@ __host__ __device__ constexpr int plan_radix_dir(int L, int q, bool rev, int pol
     return rev ? plan_radix(L, plan_len(L, policy) - 1 - q, policy) : plan_radix(L, q, policy);
 }
 
-// largest radix used by the plan of L (sets the register footprint)
-__host__ __device__ constexpr int max_radix(int L, int policy = 0) {
-    int m = 1;
-    bool first = true;
-    for (int rem = L; rem > 1;) {
-        const int r = pick_radix_p(L, rem, first, policy);
-        if (r == 0) return 0;
-        m = r > m ? r : m;
-        rem /= r;
-        first = false;
-    }
-    return m;
-}
-
 // Exact mathematical constants used by the radix-3/5/8 butterflies.
 #define IFDDA_SQRT3_2 0.86602540378443864676372317075294
 #define IFDDA_SQRT1_2 0.70710678118654752440084436210485
@@ -501,8 +487,9 @@ template <class Lay> constexpr bool write_split(int NJ, int Ns, int R) {
 // that writes the tile ends in a barrier (otherwise the caller's next one does).
 template <class C, int L, int R, int Ns, int NB, int NT, int DIR, class Lay, class Src, class Dst, bool SYNC = true>
 __device__ __forceinline__ void stockham_pass(C* sm, const typename elem_traits<C>::W* tw, const Src& src,
-                                              const Dst& dst, const int tid) {
+                                              const Dst& dst) {
     using W = typename elem_traits<C>::W;
+    const int tid = threadIdx.x;
     constexpr int NJ = L / R;
     constexpr int NBF = NB * NJ;
     constexpr int PER = (NBF + NT - 1) / NT;
@@ -583,25 +570,16 @@ __device__ __forceinline__ void stockham_pass(C* sm, const typename elem_traits<
 }
 
 // Passes q in [q, Q1) of the plan (reversed when REV); Ns is the product of
-// the radices of the passes before q.  tid is the thread's index; a caller
-// that loops passes it through loop_tid() below, so that the compiler does not
-// keep every twiddle and tile address of the loop body in registers.
+// the radices of the passes before q.
 template <class C, int L, int NB, int NT, int DIR, class Lay, bool REV, int Q1, int q, int Ns, class Src, class Dst,
           int PLAN = 0>
 __device__ __forceinline__ void stockham_range(C* sm, const typename elem_traits<C>::W* tw, const Src& src,
-                                               const Dst& dst, const int tid = threadIdx.x) {
+                                               const Dst& dst) {
     if constexpr (q < Q1) {
         constexpr int R = plan_radix_dir(L, q, REV, PLAN);
-        stockham_pass<C, L, R, Ns, NB, NT, DIR, Lay, Src, Dst>(sm, tw, src, dst, tid);
-        stockham_range<C, L, NB, NT, DIR, Lay, REV, Q1, q + 1, Ns * R, Src, Dst, PLAN>(sm, tw, src, dst, tid);
+        stockham_pass<C, L, R, Ns, NB, NT, DIR, Lay, Src, Dst>(sm, tw, src, dst);
+        stockham_range<C, L, NB, NT, DIR, Lay, REV, Q1, q + 1, Ns * R, Src, Dst, PLAN>(sm, tw, src, dst);
     }
-}
-
-// threadIdx.x as a value the compiler takes to change from iteration to iteration
-__device__ __forceinline__ int loop_tid() {
-    int t = threadIdx.x;
-    asm volatile("" : "+r"(t));
-    return t;
 }
 
 // Transform NB lines.  When the source is shared memory the caller must have

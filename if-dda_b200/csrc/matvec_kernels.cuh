@@ -524,10 +524,6 @@ __device__ __forceinline__ cpair gfma2(cpair acc, float2 g0, float2 g1, float s,
 __device__ __forceinline__ float2 flip(float2 v, unsigned f) {
     return make_float2(__uint_as_float(__float_as_uint(v.x) ^ f), __uint_as_float(__float_as_uint(v.y) ^ f));
 }
-__device__ __forceinline__ double2 flip(double2 v, unsigned f) {
-    return make_double2(__hiloint2double(__double2hiint(v.x) ^ (int)f, __double2loint(v.x)),
-                        __hiloint2double(__double2hiint(v.y) ^ (int)f, __double2loint(v.y)));
-}
 
 // v <- G v for the RK points j + r NJ of one column; g: its slice [c6][qz].
 // Spectral mirrors: z beyond nz flips xz and yz, the row Y - qy xy and yz
@@ -547,8 +543,11 @@ __device__ __forceinline__ void zmultiply(E (&v)[3][RK], const W* g, unsigned my
         const W* gq = g + (mir ? L - p : p);
         const T sz = mir ? T(-1) : T(1);
         const E x = v[0][r], y = v[1][r], z = v[2][r];
-        const W gxy = MY < 0 ? flip(gq[NQ], my) : gq[NQ], gxz = gq[2 * NQ];
-        const W gyz = MY < 0 ? flip(gq[4 * NQ], my) : gq[4 * NQ];
+        W gxy = gq[NQ], gxz = gq[2 * NQ], gyz = gq[4 * NQ];
+        if constexpr (MY < 0) {
+            gxy = flip(gxy, my);
+            gyz = flip(gyz, my);
+        }
         v[0][r] = gfma(gfma(gmul(gq[0], x), gxy, sy, y), gxz, sz, z);
         v[1][r] = gfma(gfma(gmul(gq[3 * NQ], y), gxy, sy, x), gyz, sy * sz, z);
         v[2][r] = gfma(gfma(gmul(gq[5 * NQ], z), gxz, sz, x), gyz, sy * sz, y);
@@ -658,8 +657,7 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
     const ZLoad<E, TL, TT::ZPF> zload{B2, rs, comp, nv};
     const ZStore<E, TL> zstore{B2, rs, comp, nv};
     if constexpr (NP > 1) {
-        stockham_pass<E, L, TT::RZ, 1, NB, NT, +1, LZ, ZLoad<E, TL, TT::ZPF>, SmemIO, false>(sm, tw, zload, SmemIO{},
-                                                                                           threadIdx.x);
+        stockham_pass<E, L, TT::RZ, 1, NB, NT, +1, LZ, ZLoad<E, TL, TT::ZPF>, SmemIO, false>(sm, tw, zload, SmemIO{});
         if constexpr (!TT::ZSMALL && NP == 2) cp_async_wait_all();
         __syncthreads();
         stockham_range<E, L, NB, NT, +1, LZ, false, NP - 1, 1, TT::RZ, SmemIO, SmemIO, TT::PZ>(sm, tw, SmemIO{},
