@@ -773,9 +773,10 @@ int ifdda_inverserig_batch(ifdda_green* g, int nrhs, int nbsphere, int nmax, con
     const int* tab = nullptr;
     if (tabdip) check_tabdip(tabdip, uN, nbsphere);
     // The inputs are uploaded on the context's upload stream when their
-    // buffers need no allocation, so that the copies overlap the work already
-    // queued on the solve stream (in the reference's call sequence the
-    // spectrum, cdmlib/cdmlib.f:1529, comes right before the solve, :1565);
+    // buffers need no allocation, so that the copies overlap work that the
+    // caller has queued on the solve stream without waiting for it (a mat-vec
+    // or a solve on device arrays; after the spectrum, cdmlib/cdmlib.f:1529,
+    // the stream is idle, since ifdda_green_recompute returns when it is done);
     // the solve stream waits for them (upload_done) before the solve.  A
     // buffer that must grow is allocated and filled on the solve stream,
     // after the upload stream has drained (a pending upload may still target

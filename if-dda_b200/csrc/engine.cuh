@@ -23,6 +23,11 @@
 
 namespace ifdda {
 
+// the kernels' element offsets are ints (see FwdXLoad)
+#define IFDDA_INT_OFFSETS(L) static_assert(3LL * (L / 2) * L * L < (1LL << 31), "element offsets of length " #L);
+IFDDA_FFT_LENGTHS(IFDDA_INT_OFFSETS)
+#undef IFDDA_INT_OFFSETS
+
 bool fft_length_supported(int L);
 
 struct EngineError {
@@ -127,9 +132,8 @@ struct TileChoice {
 // Tile chooser results, one per (device, precision 0 FP64 / 1 FP32, grid
 // X x Y x Z), shared by every spectrum on that grid and every batch size: a
 // request stream of many spectra on few grids times each grid once, and a
-// right-hand side runs the same kernels alone and in a batch (the shapes can
-// differ in the last bits where the compiler contracts multiply-adds
-// differently, so one grid keeps one shape).
+// right-hand side runs the same kernels alone and in a batch (the shapes differ
+// in the last bits where they take other plans, so one grid keeps one shape).
 bool tile_get(int dev, int prec, const MvGeom& g, TileChoice& out);
 void tile_put(int dev, int prec, const MvGeom& g, const TileChoice& tc);
 void tile_erase(int dev, int prec, const MvGeom& g);

@@ -98,9 +98,13 @@ template <class T> struct MvArgs {
 //    columns (8 x 8 x 8, 8 right-hand sides: 8.6 us a product against 9.0 with
 //    8 and 9.2 with 32), and 32 up to length 8 (64 x 2 x 64 in FP64 17.8 us
 //    with 8, 14.6 with 16, 13.2 with 32);
-//  * zconv: 8 columns of 16 bytes, rows of 128 bytes.  4 columns (V = 1 below
-//    160) and 2 give more and smaller blocks, but their narrower rows cost more
-//    than that: FP64 at 64^3 43.5, 47.5 and 65 us, FP32 27.9, 29.5 and 40.5 us.
+//  * zconv: 8 columns of 16 bytes, rows of 128 bytes, from length 12 to 160.  4
+//    columns (V = 1 from length 12 to 128) and 2 give more and smaller blocks,
+//    but their narrower rows cost more than that: FP64 at 64^3 43.5, 47.5 and
+//    65 us, FP32 27.9, 29.5 and 40.5 us.  Longer columns no longer fit 112 KB, so
+//    that two blocks share an SM: V = 0 takes 4 at 192 and 256 (FP32 also at
+//    320) and 2 beyond; V = 1, without the spectrum in shared memory, 8 up to 256,
+//    4 at 320 and 384 (FP32 also at 512) and 2 beyond.
 //    From 160 on two passes need 150 to 250 registers a thread, which leaves 6
 //    to 12 warps per SM; there V = 1 takes three passes of small radices at 80
 //    registers and reads the spectrum where it uses it (L2), so that 24 warps
@@ -122,7 +126,11 @@ template <class T> struct MvArgs {
 // need (128x128x2 x4 in FP64 45.9 us with 84, which spills, 42.8 with 102 or 128).
 // The variants are compiled for lengths of 64 and more; the tile chooser
 // (tune_tiles) times both on the caller's grid and keeps one per grid.  The
-// two agree to rounding.
+// two agree to rounding.  Below length 160 V = 1 is for lattices whose wider
+// tiles leave SMs without a block: products of 16x32x32 13.3 -> 12.3 us (FP32
+// 11.5 -> 10.8), 32^3 in FP32 13.8 -> 12.6, 1x64x64 14.2 -> 11.8 (FP32 13.2 ->
+// 12.2); from 40^3 or from several right-hand sides on V = 0 is as good or
+// better (64^3 80.0 against 85.5 us, FP32 43.7 against 45.5).
 //
 // Tried without gain and left out: B2 stored in column tiles (z rows no longer
 // a power of two apart), a persistent zconv that copies the next row's input
@@ -250,9 +258,11 @@ template <class T> struct PreNone {
 };
 
 // Element offsets inside one right-hand side's vectors and scratch fit in 32
-// bits for every compiled FFT length (at most 3 * 192^3 dipole components,
-// 3 * 192 * 384^2 grid points), so the pass functors index with int from
-// per-block base pointers; the fields they need are copied by value.
+// bits for every compiled FFT length L (at most 3 (L/2)^3 dipole components
+// and 3 (L/2) L^2 grid points, 3.9e8 at length 640; checked where the lengths
+// are listed), and so do those of a full polarisability tensor of up to 2^31 / 9
+// dipoles, so the pass functors index with int from per-block base pointers;
+// the fields they need are copied by value.
 template <class T, bool TAB, class Pre> struct FwdXLoad {
     static constexpr bool GLOBAL = true, HALF = true;  // points p >= nx are the padding
     const int* tab;
