@@ -38,14 +38,21 @@ template <int L> struct GreenTiles {
     static constexpr int TLX = clamp_pow2(49152 / (L * 6 * S), 1, 8);
     static constexpr int TLY = clamp_pow2(49152 / (L * S), 2, 16);
     static constexpr int NT = 256;
+    // Blocks per SM asked of the compiler where it otherwise takes a few
+    // registers too many for them: the x pass at 384 (83 registers, two blocks;
+    // 192^3 998 us instead of 784) and 512, the y pass at 320 (160x160x64 234
+    // instead of 179) and at 96 (52 registers).
+    static constexpr int MINBX = L == 384 || L == 512 ? 3 : 0;  // 0: the compiler's choice
+    static constexpr int minb(int axis) { return axis == 2 ? 0 : L == 320 ? 3 : L == 96 ? 5 : 0; }
     static constexpr int LSX = (6 * TLX) | 1;
     static constexpr size_t smem_x = (size_t)L * S + (size_t)L * LSX * S;
     // Columns of a block of the y and of the z pass: 32 in the z pass up to
     // length 48 (16: 256x256x5 163 us instead of 147).  The z pass, which reads
-    // its lines point by point to write them, has one column of padding; the y
-    // pass has none (with it the spectrum of 64x80x64 took 147 us instead of 128).
+    // its lines point by point to write them, has one column of padding where a
+    // row fills the banks; the y pass has none (with it the spectrum of 64x80x64
+    // took 147 us instead of 128).
     static constexpr int tl(int axis) { return axis == 1 || L > 48 ? TLY : clamp_pow2(49152 / (L * S), 2, 32); }
-    static constexpr int ls(int axis) { return axis == 1 ? tl(1) : tl(2) + 1; }
+    static constexpr int ls(int axis) { return axis == 1 || tl(2) < 8 ? tl(axis) : tl(2) + 1; }
     static constexpr size_t smem_yz(int axis) { return (size_t)L * S + (size_t)L * ls(axis) * S; }
 };
 
@@ -167,7 +174,7 @@ __device__ __forceinline__ double green_py(int c) { return (c == 1 || c == 4) ? 
 __device__ __forceinline__ double green_pz(int c) { return (c == 2 || c == 4) ? -1.0 : 1.0; }
 
 template <int L>
-__global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_x(const GreenGeom g, double2* __restrict__ GA,
+__global__ void __launch_bounds__(GreenTiles<L>::NT, GreenTiles<L>::MINBX) k_green_x(const GreenGeom g, double2* __restrict__ GA,
                                                                const double2* __restrict__ twx) {
     using C = double2;
     using TT = GreenTiles<L>;
@@ -208,7 +215,7 @@ __global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_x(const GreenGeom g
 // Py(c) times row Y - y;  AXIS 2: GB -> Gc[ny+1][W][c][nz+1], planes z > nz
 // read as Pz(c) times plane Z - z
 template <int L, int AXIS>
-__global__ void __launch_bounds__(GreenTiles<L>::NT) k_green_yz(const GreenGeom g, const double2* __restrict__ src,
+__global__ void __launch_bounds__(GreenTiles<L>::NT, GreenTiles<L>::minb(AXIS)) k_green_yz(const GreenGeom g, const double2* __restrict__ src,
                                                                 double2* __restrict__ dst64, float2* __restrict__ dst32,
                                                                 const double2* __restrict__ tw_axis) {
     using C = double2;
