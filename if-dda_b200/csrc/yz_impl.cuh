@@ -58,9 +58,11 @@ template <class T> void launch_yz_impl(const MvArgs<T>& a, int nrhs, cudaStream_
 // tile variant of the y passes (forward then inverse) and of zconv, best of
 // three launches with CUDA events on st, and record the choice for G's grid,
 // device and precision (tile_put: every spectrum and batch size on that grid
-// then uses it).  Variant 1 is taken only when it is at least 5% faster, so
-// timing noise between near-equal shapes does not flip the choice.  Never
-// runs while st is being captured.
+// then uses it).  Variant 0 is the one to beat by 5%, so that timing noise
+// between near-equal shapes does not flip the choice; where a row does not
+// half fill its tile (nx up to 8 in the y passes, 4 in zconv, in FP32; half
+// that in FP64), variant 1 is (products of 1x64x64 in FP32 13.3 -> 12.6 us,
+// 2x64x64 in FP64 15.9 -> 12.7).  Never runs while st is being captured.
 template <class T> void tune_tiles_impl(Green& G, int nrhs, cudaStream_t st) {
     const int pk = sizeof(T) == 4 ? 1 : 0;
     TileChoice have;
@@ -71,6 +73,9 @@ template <class T> void tune_tiles_impl(Green& G, int nrhs, cudaStream_t st) {
     MvArgs<T> a = mv_args<T>(G, nrhs, nullptr, nullptr, nullptr, 0, ALPHA_NONE, nullptr, 0, nullptr, nullptr);
     TileChoice tc{};
     const int nyv = tile_variants(G.g.Y), nzv = tile_variants(G.g.Z);
+    const int columns = G.g.X * (int)sizeof(cplx<T>) / (int)sizeof(typename yz_elem<T>::type);
+    tc.yvar = nyv > 1 && columns <= 8 ? 1 : 0;
+    tc.zvar = nzv > 1 && G.g.Z < 160 && columns <= 4 ? 1 : 0;
     if (nyv > 1 || nzv > 1) {
         cudaEvent_t e0, e1;
         IFDDA_CUDA(cudaEventCreate(&e0));
@@ -93,15 +98,15 @@ template <class T> void tune_tiles_impl(Green& G, int nrhs, cudaStream_t st) {
             tc.y_ms[v] = time_it([&] {
                 switch (G.g.Y) { IFDDA_FFT_LENGTHS(IFDDA_CASE_TY) default: break; }
             });
-            if (tc.y_ms[v] < 0.95f * tc.y_ms[tc.yvar]) tc.yvar = v;
         }
+        if (nyv > 1 && tc.y_ms[1 - tc.yvar] < 0.95f * tc.y_ms[tc.yvar]) tc.yvar = 1 - tc.yvar;
         for (int v = 0; v < nzv; v++) {
             a.zvar = v;
             tc.z_ms[v] = time_it([&] {
                 switch (G.g.Z) { IFDDA_FFT_LENGTHS(IFDDA_CASE_TZ) default: break; }
             });
-            if (tc.z_ms[v] < 0.95f * tc.z_ms[tc.zvar]) tc.zvar = v;
         }
+        if (nzv > 1 && tc.z_ms[1 - tc.zvar] < 0.95f * tc.z_ms[tc.zvar]) tc.zvar = 1 - tc.zvar;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     }
