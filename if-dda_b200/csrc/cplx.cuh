@@ -23,7 +23,7 @@ namespace ifdda {
 // starts.  Triggering first instead lets a whole chain of waiting kernels
 // occupy the SMs, and the blocks of a small grid then land where there is
 // room, several on one SM: a product on 24^3 in FP64 took 19.8 instead of
-// 12.7 us, one on 32^3 in FP32 21.7 instead of 15.2 us (64^3: no difference).
+// 12.8 us, one on 32^3 in FP32 21.7 instead of 14.0 us (64^3: no difference).
 // A kernel whose vectors the next one reads through the read-only path (ldg)
 // triggers after it has written them, so that they do not change while the
 // reader runs.  The reader's early return of a finished solve stands between

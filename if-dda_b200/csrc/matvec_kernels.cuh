@@ -594,8 +594,8 @@ __device__ __forceinline__ void zmultiply_ends(cpair (&v)[3][RK], const float2* 
 // Bound by latency at 12 warps per SM: at 64^3 the FP64 pipe, shared memory and
 // instruction issue are each 35-40% busy.  Against one complex value per
 // thread and element, a slice of the spectrum per column and 2.06e7 warp
-// instructions: FP64 58.1 -> 43.5 us (1.60e7), FP32 35.2 -> 27.9 us (1.95e7 ->
-// 1.06e7: packed sums, one spectrum value for two columns, no work on the
+// instructions: FP64 58.1 -> 42.9 us (1.54e7), FP32 35.2 -> 26.9 us (1.95e7 ->
+// 0.98e7: packed sums, one spectrum value for two columns, no work on the
 // padding's zeros).
 // Grid (2 right-hand side + mirror row, column tile, qy): the blocks that read
 // one slice of the spectrum run together, so a batch takes that slice from
