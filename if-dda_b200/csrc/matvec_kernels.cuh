@@ -99,7 +99,7 @@ template <class T> struct MvArgs {
 //    8 and 9.2 with 32), and 32 up to length 8 (64 x 2 x 64 in FP64 17.8 us
 //    with 8, 14.6 with 16, 13.2 with 32);
 //  * zconv: 8 columns of 16 bytes, rows of 128 bytes, from length 12 to 160.  4
-//    columns (V = 1 from length 12 to 128) and 2 give more and smaller blocks,
+//    columns (V = 1 from length 64 to 128) and 2 give more and smaller blocks,
 //    but their narrower rows cost more than that: FP64 at 64^3 43.5, 47.5 and
 //    65 us, FP32 27.9, 29.5 and 40.5 us.  Longer columns no longer fit 112 KB, so
 //    that two blocks share an SM: V = 0 takes 4 at 192 and 256 (FP32 also at
@@ -114,8 +114,8 @@ template <class T> struct MvArgs {
 //    Up to length 8 a column is one thread's, with no shared memory in
 //    between, and a block takes 32 columns (64 at length 2), at length 10 16:
 //    with 8 columns and two passes most threads had no work.  Product of
-//    256x256x1 in FP64 66.1 -> 33.7 us, 128x128x2 x4 70.4 -> 44.9, 128x128x4 x2
-//    55.2 -> 43.8, 256x256x5 192.7 -> 130.9; in FP32 37.5 -> 25.0, 42.4 -> 31.2,
+//    256x256x1 in FP64 66.1 -> 33.7 us, 128x128x2 x4 70.4 -> 43.0, 128x128x4 x2
+//    55.2 -> 43.8, 256x256x5 192.7 -> 130.9; in FP32 37.5 -> 25.0, 42.4 -> 30.0,
 //    33.9 -> 30.9, 97.4 -> 67.0.
 // Register caps of the y passes and of zconv's small middles (RK up to 5): 102
 // (five warps per quarter SM; 84 for first radices up to 8 and at length 20)
