@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(TT::NTZ, TT::MINBZ) k_zconv(const MvArgs<T> a)
         static_assert(6 * TT::NQ * sizeof(W) % 16 == 0 && GST * sizeof(W) % 16 == 0, "16-byte copies");
         const char* src = reinterpret_cast<const char*>(gbase + (long)t0 * (6 * TT::NQ));
         char* dst = reinterpret_cast<char*>(gs);
-        if constexpr (CH < NT) {  // several columns at a time
+        if constexpr (2 * CH <= NT) {  // several columns at a time
             for (int e = threadIdx.x; e < min(TC, nx - t0) * CH; e += NT)
                 cp_async16(dst + e / CH * (GST * (int)sizeof(W)) + e % CH * 16, src + 16 * e);
             if (t0 == 0 && (int)threadIdx.x < CH)
